@@ -176,7 +176,7 @@ def kernel_bounds(kernel_ms, counters, ceilings, clocks, samples):
     e = out.get("emission")
     if e:
         sec = e["ms"] / 1e3
-        per = (ipc or {}).get("march_spectral<4,1,shade>", {}).get("warp_inst_per_sample")
+        per = (ipc or {}).get("march_shade_spectral<4,1>", {}).get("warp_inst_per_sample")
         if per:
             e["issue"] = {"achieved": per * samples / sec, "peak": issue_peak, "frac": per * samples / sec / issue_peak,
                           "unit": "warp instructions/s", "per_sample": per}
@@ -574,7 +574,7 @@ def run_ours(args):
                                    "(overflowing segments) + march_far (far samples of wide-box views; an empty "
                                    "list here) + march_deferred (the samples the search leaves) + "
                                    "march_hard (deferred samples over the one-lane budget) + "
-                                   "march_spectral<4,1,shade> (emission from the positions), timed together",
+                                   "march_shade_spectral<4,1> (emission from the positions), timed together",
                          "binding": binding_bound(kernels)},
             "cpu_baseline": cpu,
             "autotuned": tuned,

@@ -9,7 +9,7 @@
 // each), march_hard (deferred samples over
 // a lane's budget, one warp each) -- the last four store the neighbours they
 // find in the same buffer -- and then the
-// emission pass, march_spectral<.., shade> or march_imaging<.., shade>, which
+// emission pass, march_shade_spectral or march_shade_imaging, which
 // bins every ray from the buffer.  The no-allocation path has no buffer: its
 // first pass (march_spectral / march_imaging, fused) searches and bins, and
 // the split, deferred and hard passes add their samples' emission with
@@ -936,7 +936,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // ---------------------------------------------------------------------------
 // Search pass of the two-pass spectral march: each sample's neighbour (sorted
 // position, -1 for none or deferred) into a.npos, [work item - item_base][k],
-// streamed past L2; the NN indices when asked for.  march_spectral<.., true>
+// streamed past L2; the NN indices when asked for.  march_shade_spectral
 // then bins the emission from these positions.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads, kMinCtasSearch) march_search(MarchArgs a, const double3* __restrict__ ktab,
@@ -970,19 +970,18 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSearch) march_search(MarchAr
 // Spectroscopic march: NL lines x up to NB 32-bin windows per line; lane
 // `lane` owns bins wstart + 32 m + lane of each line.
 // ---------------------------------------------------------------------------
-// SHADE: the neighbours come from the position buffer written by
-// march_search (a.npos) instead of the search itself; the emission code and
-// its arithmetic are the same.
-template <int NL, int NB, bool SHADE>
-__global__ void __launch_bounds__(kThreads, SHADE ? kMinCtasShade : kMinCtas)
+// The fused first pass of the no-allocation path: each segment is searched and
+// binned at once.
+template <int NL, int NB>
+__global__ void __launch_bounds__(kThreads, kMinCtas)
     march_spectral(MarchArgs a, const double3* __restrict__ ktab, int ktab_stride) {
-  __shared__ SegSmem segs[SHADE ? 1 : kWarps];
+  __shared__ SegSmem segs[kWarps];
   __shared__ float4 runs[kWarps][32][NL];  // a chunk's runs: (peak x length, 2/w, Doppler term) per line
   const int w = threadIdx.x >> 5;
-  SegSmem& sm = segs[SHADE ? 0 : w];
+  SegSmem& sm = segs[w];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, r, SHADE ? kCtrShade : kCtrRays)) {
+  while (next_ray(a, ktab, ktab_stride, r)) {
     const ViewDesc* V = a.views + r.v;
     const int nz = V->nz, L = V->L, nx = V->nx;
     const float ux = V->ux, uy = V->uy, uz = V->uz;
@@ -1009,18 +1008,11 @@ __global__ void __launch_bounds__(kThreads, SHADE ? kMinCtasShade : kMinCtas)
         lam[l][m] = (m < nw[l] && il < L) ? __ldg(LD[l].lam + FOMO_IDX(il, L, kSiteLam)) : 3.0e30f;
       }
     }
-    int32_t* nnout = (!SHADE && a.nn_idx) ? a.nn_idx[r.v] : nullptr;
+    int32_t* nnout = a.nn_idx ? a.nn_idx[r.v] : nullptr;
     const int64_t ray = (int64_t)r.i * nx + r.j;
-    const int32_t* npos = SHADE ? a.npos + ((int64_t)r.item - a.item_base) * ktab_stride : nullptr;
     for (int s0 = 0; s0 < nz; s0 += kSeg) {
       int posv[2], origv[2];
-      if (SHADE) {
-        posv[0] = s0 + lane < nz ? __ldcs(a.npos + FOMO_IDX(npos - a.npos + s0 + lane, a.npos_cap, kSiteNpos)) : -1;
-        posv[1] = s0 + 32 + lane < nz ? __ldcs(a.npos + FOMO_IDX(npos - a.npos + s0 + 32 + lane, a.npos_cap, kSiteNpos))
-                                      : -1;
-      } else {
-        segment_search(a, r, s0, nz, sm, posv, origv);
-      }
+      segment_search(a, r, s0, nz, sm, posv, origv);
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         const int k = s0 + 32 * h + lane;
@@ -1115,19 +1107,17 @@ __global__ void __launch_bounds__(kThreads, SHADE ? kMinCtasShade : kMinCtas)
 // ---------------------------------------------------------------------------
 // Imaging (L == 1, broadband channels) and Thomson pB: per-sample values,
 // reduced across the warp per 32-sample chunk, Kahan-accumulated per ray.
-// SHADE: the neighbours come from the position buffer (a.npos), in which the
-// search, split, deferred and hard passes have stored every sample's
-// neighbour; otherwise (the no-allocation path) the kernel searches itself and
-// the deferred samples are added by the later passes.
+// The fused first pass of the no-allocation path: the kernel searches itself
+// and the deferred samples are added by the later passes.
 // ---------------------------------------------------------------------------
-template <int NL, bool THOMSON, bool SHADE>
-__global__ void __launch_bounds__(kThreads, SHADE ? kMinCtasShade : kMinCtasImaging)
+template <int NL, bool THOMSON>
+__global__ void __launch_bounds__(kThreads, kMinCtasImaging)
     march_imaging(MarchArgs a, const double3* __restrict__ ktab, int ktab_stride) {
-  __shared__ SegSmem segs[SHADE ? 1 : kWarps];
-  SegSmem& sm = segs[SHADE ? 0 : (threadIdx.x >> 5)];
+  __shared__ SegSmem segs[kWarps];
+  SegSmem& sm = segs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, r, SHADE ? kCtrShade : kCtrRays)) {
+  while (next_ray(a, ktab, ktab_stride, r)) {
     const ViewDesc* V = a.views + r.v;
     const int nz = V->nz, nx = V->nx;
     const LineDesc* LD = a.lines + (int64_t)r.v * a.nlines;
@@ -1140,18 +1130,11 @@ __global__ void __launch_bounds__(kThreads, SHADE ? kMinCtasShade : kMinCtasImag
       lon[l] = l < a.nlines && LD[l].out != nullptr;  // views may have fewer lines than the launch
     }
     const float* s2v = THOMSON ? a.s2 + (int64_t)r.v * a.snap.n : nullptr;
-    int32_t* nnout = (!SHADE && a.nn_idx) ? a.nn_idx[r.v] : nullptr;
+    int32_t* nnout = a.nn_idx ? a.nn_idx[r.v] : nullptr;
     const int64_t ray = (int64_t)r.i * nx + r.j;
-    const int32_t* npos = SHADE ? a.npos + ((int64_t)r.item - a.item_base) * ktab_stride : nullptr;
     for (int s0 = 0; s0 < nz; s0 += kSeg) {
       int posv[2], origv[2];
-      if (SHADE) {
-        posv[0] = s0 + lane < nz ? __ldcs(a.npos + FOMO_IDX(npos - a.npos + s0 + lane, a.npos_cap, kSiteNpos)) : -1;
-        posv[1] = s0 + 32 + lane < nz ? __ldcs(a.npos + FOMO_IDX(npos - a.npos + s0 + 32 + lane, a.npos_cap, kSiteNpos))
-                                      : -1;
-      } else {
-        segment_search(a, r, s0, nz, sm, posv, origv);
-      }
+      segment_search(a, r, s0, nz, sm, posv, origv);
 #pragma unroll 1
       for (int h = 0; h < 2; ++h) {
         const int k = s0 + 32 * h + lane;
@@ -1185,6 +1168,269 @@ __global__ void __launch_bounds__(kThreads, SHADE ? kMinCtasShade : kMinCtasImag
         if (lon[l])
           LD[l].out[FOMO_IDX(ray, (int64_t)nx * V->ny, kSiteCube)] =
               __double2float_rn(__dmul_rn(LD[l].is_dn ? V->scale_dn : V->scale, (double)acc[l]));
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Emission pass: every ray's neighbours come from the position buffer (a.npos),
+// in which the search, split, far, deferred and hard passes have stored them;
+// one warp bins one ray.
+//
+// What bounds it is the gather of each run's payload (velocity, and width and
+// peak per line): scattered 8- and 16-byte loads from L2.  A run of equal
+// neighbours is 5 samples long on the 2M-point loop at 512 samples, so a
+// warp's 32 samples hold 6 of them: gathering chunk by chunk left 26 lanes idle
+// through every load, reciprocal and staging step.  Here the run starts of the
+// whole ray go to a ring in shared memory first, and the payloads are gathered
+// when 32 runs are pending, one per lane.  A run may span chunks, so there
+// are also fewer of them.  64 views x 4 lines of 256 x 256 x 512 samples: 32.4 ms
+// chunk by chunk, 18.0 now (issue 74 %, L1 70 %); 6 channels of 1024 x 1024 x
+// 1024: 7.6 -> 3.5 ms.
+// ---------------------------------------------------------------------------
+constexpr int kRunAhead = 4;   // chunks of 32 neighbours loaded together
+constexpr int kRunRing = 256;  // pending runs: at most 32 left over and 32 kRunAhead new ones
+struct RunRing {
+  int pos[kRunRing];  // neighbour of the run (sorted position, -1 for none)
+  int k[kRunRing];    // its first sample
+};
+
+// Warp-collective: the runs of equal neighbours of one ray, in sample order.
+// batch(m, pos, len) is called by the whole warp for up to 32 runs at a time:
+// lane i < m holds run i (pos -1: samples without a neighbour); m is 32 but
+// for the ray's last batch.
+template <typename F>
+__device__ __forceinline__ void walk_runs(const MarchArgs& a, const RayCtx& r, int ktab_stride, RunRing& ring, F&& batch) {
+  const int lane = threadIdx.x & 31;
+  const int nz = r.nz;
+  const int64_t row = ((int64_t)r.item - a.item_base) * ktab_stride;
+  const unsigned lt = (1u << lane) - 1u;
+  int head = 0, tail = 0, carry = -3;  // carry: the neighbour before the chunk
+  for (int s0 = 0; s0 < nz; s0 += 32 * kRunAhead) {
+    int p[kRunAhead];
+#pragma unroll
+    for (int u = 0; u < kRunAhead; ++u) {
+      const int k = s0 + 32 * u + lane;
+      p[u] = k < nz ? __ldcs(a.npos + FOMO_IDX(row + k, a.npos_cap, kSiteNpos)) : -2;
+    }
+#pragma unroll
+    for (int u = 0; u < kRunAhead; ++u) {
+      const int k = s0 + 32 * u + lane;
+      const int up = __shfl_up_sync(kFull, p[u], 1);
+      const bool start = k < nz && p[u] != (lane == 0 ? carry : up);
+      carry = __shfl_sync(kFull, p[u], 31);
+      const unsigned starts = __ballot_sync(kFull, start);
+      if (start) {
+        const int slot = (tail + __popc(starts & lt)) & (kRunRing - 1);
+        ring.pos[slot] = p[u];
+        ring.k[slot] = k;
+      }
+      tail += __popc(starts);
+    }
+    __syncwarp();
+    const bool last = s0 + 32 * kRunAhead >= nz;
+    while (tail - head > 32 || (last && tail > head)) {  // the 33rd start ends the 32nd run
+      const int m = min(32, tail - head), i = head + lane;
+      const int pos = lane < m ? ring.pos[i & (kRunRing - 1)] : -1;
+      const int k = lane < m ? ring.k[i & (kRunRing - 1)] : 0;
+      const int next = i + 1 < tail ? ring.k[(i + 1) & (kRunRing - 1)] : nz;
+      head += m;
+      batch(m, pos, next - k);
+    }
+  }
+  __syncwarp();  // the ring is rewritten by the next ray
+}
+
+// Spectroscopy: NL lines x up to NB 32-bin windows per line.  The batch's runs
+// are staged as (peak x length, 2/w, Doppler term) per line, compacted to those
+// with a neighbour, and binned line by line and window by window: the warp is
+// four groups of eight lanes, group g adds runs g, g + 4, ... and each lane
+// evaluates four of the window's bins.  With one run for the whole warp, every
+// (run, line) cost a 16-byte broadcast to 32 lanes, 512 bytes through the shared-
+// memory port, which was the bound (22.7 ms, L1 at 85 %); a load now serves four
+// runs (18.0 ms).
+// The groups' sums are joined by an exchange that leaves bin `lane` in each
+// lane, and folded into the ray's Kahan sum.
+template <int NL, int NB>
+__global__ void __launch_bounds__(kThreads, kMinCtasShade)
+    march_shade_spectral(MarchArgs a, const double3* __restrict__ ktab, int ktab_stride) {
+  __shared__ RunRing rings[kWarps];
+  __shared__ float4 runs[kWarps][NL][32];
+  __shared__ float lams[kWarps][NL][NB * 32];  // lambdaval (nn:200), evaluated in FP64 on the host, stored FP32
+  const int w = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int group = lane >> 3;
+  RayCtx r;
+  int view = -1;
+  while (next_ray(a, ktab, ktab_stride, r, kCtrShade)) {
+    const ViewDesc* V = a.views + r.v;
+    const int L = V->L, nx = V->nx;
+    const float ux = V->ux, uy = V->uy, uz = V->uz;
+    const LineDesc* LD = a.lines + (int64_t)r.v * a.nlines;
+    float acc[NL][NB], comp[NL][NB], shk[NL];
+    const float2* ew[NL];
+    int nw[NL];  // windows of the line; 0: the view has fewer lines than the launch
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      const bool on = l < a.nlines && LD[l].ew != nullptr;
+      ew[l] = on ? LD[l].ew : nullptr;
+      shk[l] = on ? LD[l].shift_k : 0.0f;
+      nw[l] = on ? min(LD[l].nw, NB) : 0;
+#pragma unroll
+      for (int m = 0; m < NB; ++m) {
+        acc[l][m] = 0.0f;
+        comp[l][m] = 0.0f;
+        if (r.v != view && m < nw[l]) {
+          const int il = LD[l].wstart + m * 32 + lane;
+          lams[w][l][m * 32 + lane] = il < L ? __ldg(LD[l].lam + FOMO_IDX(il, L, kSiteLam)) : 3.0e30f;
+        }
+      }
+    }
+    view = r.v;
+    walk_runs(a, r, ktab_stride, rings[w], [&](int m, int pos, int len) {
+      const unsigned fills = __ballot_sync(kFull, lane < m && pos >= 0);
+      const int nruns = __popc(fills);
+      if (!nruns) return;
+      const int npad = (nruns + 3) & ~3;
+      if (lane < m && pos >= 0) {
+        const float cnt = (float)len;
+        const float4 vv = __ldg(a.snap.vel + FOMO_IDX(pos, a.snap.n, kSitePts));
+        float2 pw[NL];
+#pragma unroll
+        for (int l = 0; l < NL; ++l)
+          pw[l] = nw[l] ? __ldg(ew[l] + FOMO_IDX(pos, a.snap.n, kSitePts)) : make_float2(0.0f, 1.0f);
+        const float vlos = fmaf(uz, vv.z, fmaf(uy, vv.y, ux * vv.x));
+        const int d = __popc(fills & ((1u << lane) - 1u));
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          // a peak of 0 (intpolpeak ? ... : 0, nn:204) is staged as all zeros and adds nothing
+          const float sc = __fdividef(2.0f, pw[l].y);  // exp(-4 ln2 (d/w)^2) = 2^(-(2d/w)^2)
+          runs[w][l][d] = pw[l].x != 0.0f ? make_float4(pw[l].x * cnt, sc, -(vlos * shk[l]) * sc, 0.0f)
+                                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+      }
+      if (lane >= nruns && lane < npad) {
+#pragma unroll
+        for (int l = 0; l < NL; ++l) runs[w][l][lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+      __syncwarp();
+      if (a.stats && lane == 0) {
+        int nwin = 0;
+#pragma unroll
+        for (int l = 0; l < NL; ++l) nwin += nw[l];
+        atomicAdd(a.stats + kStatRuns, (unsigned long long)nruns);
+        atomicAdd(a.stats + kStatEx2, 32ull * (unsigned long long)(nruns * nwin));
+      }
+#pragma unroll
+      for (int l = 0; l < NL; ++l) {
+#pragma unroll
+        for (int m2 = 0; m2 < NB; ++m2) {
+          if (m2 >= nw[l]) break;
+          float lam[4], part[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            lam[j] = lams[w][l][m2 * 32 + 8 * j + (lane & 7)];
+            part[j] = 0.0f;
+          }
+#pragma unroll 2
+          for (int q0 = group; q0 < npad; q0 += 4) {
+            const float4 t = runs[w][l][q0];  // the same address in the group's lanes
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float q = fmaf(lam[j], t.y, t.z);
+              part[j] = fmaf(t.x, ex2_approx(-q * q), part[j]);
+            }
+          }
+          // lane 8 g + i ends with the four groups' sum of bin 8 g + i
+          const bool hi = lane & 16, mid = lane & 8;
+          const float k0 = (hi ? part[2] : part[0]) + __shfl_xor_sync(kFull, hi ? part[0] : part[2], 16);
+          const float k1 = (hi ? part[3] : part[1]) + __shfl_xor_sync(kFull, hi ? part[1] : part[3], 16);
+          kahan_add(acc[l][m2], comp[l][m2], (mid ? k1 : k0) + __shfl_xor_sync(kFull, mid ? k0 : k1, 8));
+        }
+      }
+      __syncwarp();  // the staged runs are rewritten by the next batch
+    });
+    const int64_t ray = (int64_t)r.i * nx + r.j;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      if (nw[l]) {
+        const double scale = LD[l].is_dn ? V->scale_dn : V->scale;
+        float* out = LD[l].out;
+        const int64_t ncube = (int64_t)nx * V->ny * L;
+        const int wlo = LD[l].wstart, whi = wlo + 32 * nw[l];
+        for (int il = lane; il < L; il += 32)
+          if (il < wlo || il >= whi) out[FOMO_IDX(ray * L + il, ncube, kSiteCube)] = 0.0f;  // below 2^-64 of every peak
+#pragma unroll
+        for (int m = 0; m < NB; ++m) {
+          const int il = wlo + m * 32 + lane;
+          if (m < nw[l] && il < L)
+            out[FOMO_IDX(ray * L + il, ncube, kSiteCube)] = __double2float_rn(__dmul_rn(scale, (double)acc[l][m]));
+        }
+      }
+    }
+  }
+}
+
+// Imaging (L == 1) and Thomson pB: each lane adds its runs' (value x length) to
+// its own Kahan sum per line; the lanes' sums are joined once per ray, with
+// their compensations.
+template <int NL, bool THOMSON>
+__global__ void __launch_bounds__(kThreads, kMinCtasShade)
+    march_shade_imaging(MarchArgs a, const double3* __restrict__ ktab, int ktab_stride) {
+  __shared__ RunRing rings[kWarps];
+  const int lane = threadIdx.x & 31;
+  RayCtx r;
+  while (next_ray(a, ktab, ktab_stride, r, kCtrShade)) {
+    const ViewDesc* V = a.views + r.v;
+    const LineDesc* LD = a.lines + (int64_t)r.v * a.nlines;
+    float acc[NL], comp[NL];
+    const float2* ew[NL];
+    bool lon[NL];
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      acc[l] = 0.0f;
+      comp[l] = 0.0f;
+      lon[l] = l < a.nlines && LD[l].out != nullptr;  // views may have fewer lines than the launch
+      ew[l] = lon[l] ? LD[l].ew : nullptr;
+    }
+    const float* s2v = THOMSON ? a.s2 + (int64_t)r.v * a.snap.n : nullptr;
+    walk_runs(a, r, ktab_stride, rings[threadIdx.x >> 5], [&](int m, int pos, int len) {
+      if (lane < m && pos >= 0) {
+        const float cnt = (float)len;
+        float val[NL];
+#pragma unroll
+        for (int l = 0; l < NL; ++l) {
+          val[l] = 0.0f;
+          if (THOMSON) {
+            // pB = pol * sin^2 chi, clamped at 0 (thomson:325-338)
+            val[l] = fmaxf(__ldg(a.totpol + FOMO_IDX(pos, a.snap.n, kSitePts)).y *
+                               __ldg(s2v + FOMO_IDX(pos, a.snap.n, kSiteS2)),
+                           0.0f);
+          } else if (lon[l]) {
+            val[l] = __ldg(ew[l] + FOMO_IDX(pos, a.snap.n, kSitePts)).x;  // imaging adds the peak (nn:217-225)
+          }
+        }
+#pragma unroll
+        for (int l = 0; l < NL; ++l) kahan_add(acc[l], comp[l], val[l] * cnt);
+      }
+    });
+    const int64_t ray = (int64_t)r.i * V->nx + r.j;
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+      if (!lon[l]) continue;
+      float s = acc[l], c = comp[l];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float so = __shfl_xor_sync(kFull, s, o), co = __shfl_xor_sync(kFull, c, o);
+        // s + so with its rounding error (two-sum); comp holds what a sum has too much
+        const float t = __fadd_rn(s, so), bb = __fsub_rn(t, s);
+        const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(so, bb));
+        s = t;
+        c = __fsub_rn(__fadd_rn(c, co), e);
+      }
+      if (lane == 0)
+        LD[l].out[FOMO_IDX(ray, (int64_t)V->nx * V->ny, kSiteCube)] = __double2float_rn(
+            __dmul_rn(LD[l].is_dn ? V->scale_dn : V->scale, __dsub_rn((double)s, (double)c)));
     }
   }
 }
@@ -2215,17 +2461,17 @@ cudaError_t launch_queue(K kernel, const MarchArgs& a, const double3* ktab, int 
 // search pass has stored its neighbours).
 cudaError_t launch_emission_pass(const MarchArgs& a, const double3* ktab, int ktab_stride, int max_windows,
                                  int sm_count, cudaStream_t s, bool imaging) {
-  if (a.s2) return launch_persistent(march_imaging<1, true, true>, a, ktab, ktab_stride, sm_count, s, 0);
+  if (a.s2) return launch_persistent(march_shade_imaging<1, true>, a, ktab, ktab_stride, sm_count, s, 0);
   if (imaging) {
-    if (a.nlines <= 1) return launch_persistent(march_imaging<1, false, true>, a, ktab, ktab_stride, sm_count, s, 0);
-    if (a.nlines <= 2) return launch_persistent(march_imaging<2, false, true>, a, ktab, ktab_stride, sm_count, s, 0);
-    if (a.nlines <= 4) return launch_persistent(march_imaging<4, false, true>, a, ktab, ktab_stride, sm_count, s, 0);
-    if (a.nlines <= 8) return launch_persistent(march_imaging<8, false, true>, a, ktab, ktab_stride, sm_count, s, 0);
+    if (a.nlines <= 1) return launch_persistent(march_shade_imaging<1, false>, a, ktab, ktab_stride, sm_count, s, 0);
+    if (a.nlines <= 2) return launch_persistent(march_shade_imaging<2, false>, a, ktab, ktab_stride, sm_count, s, 0);
+    if (a.nlines <= 4) return launch_persistent(march_shade_imaging<4, false>, a, ktab, ktab_stride, sm_count, s, 0);
+    if (a.nlines <= 8) return launch_persistent(march_shade_imaging<8, false>, a, ktab, ktab_stride, sm_count, s, 0);
     return cudaErrorInvalidValue;
   }
   const int nb = max_windows < 1 ? 1 : max_windows;
 #define FOMO_SHADE(NL_, NB_) \
-  if (a.nlines <= NL_ && nb <= NB_) return launch_persistent(march_spectral<NL_, NB_, true>, a, ktab, ktab_stride, sm_count, s, 0)
+  if (a.nlines <= NL_ && nb <= NB_) return launch_persistent(march_shade_spectral<NL_, NB_>, a, ktab, ktab_stride, sm_count, s, 0)
   FOMO_SHADE(1, 1);
   FOMO_SHADE(1, 2);
   FOMO_SHADE(1, 4);
@@ -2244,17 +2490,17 @@ cudaError_t launch_emission_pass(const MarchArgs& a, const double3* ktab, int kt
 // kernel (no position buffer).
 cudaError_t launch_fused_pass(const MarchArgs& a, const double3* ktab, int ktab_stride, int max_windows,
                               int sm_count, cudaStream_t s, int blocks_per_sm_hint, bool imaging) {
-  if (a.s2) return launch_persistent(march_imaging<1, true, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
+  if (a.s2) return launch_persistent(march_imaging<1, true>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
   if (imaging) {
-    if (a.nlines <= 1) return launch_persistent(march_imaging<1, false, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
-    if (a.nlines <= 2) return launch_persistent(march_imaging<2, false, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
-    if (a.nlines <= 4) return launch_persistent(march_imaging<4, false, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
-    if (a.nlines <= 8) return launch_persistent(march_imaging<8, false, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
+    if (a.nlines <= 1) return launch_persistent(march_imaging<1, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
+    if (a.nlines <= 2) return launch_persistent(march_imaging<2, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
+    if (a.nlines <= 4) return launch_persistent(march_imaging<4, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
+    if (a.nlines <= 8) return launch_persistent(march_imaging<8, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
     return cudaErrorInvalidValue;
   }
   const int nb = max_windows < 1 ? 1 : max_windows;
 #define FOMO_SPEC(NL_, NB_) \
-  if (a.nlines <= NL_ && nb <= NB_) return launch_persistent(march_spectral<NL_, NB_, false>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint)
+  if (a.nlines <= NL_ && nb <= NB_) return launch_persistent(march_spectral<NL_, NB_>, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint)
   FOMO_SPEC(1, 1);
   FOMO_SPEC(1, 2);
   FOMO_SPEC(1, 4);
