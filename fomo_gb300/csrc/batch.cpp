@@ -28,7 +28,7 @@ std::string plan_key(const Plan& p, const ScratchSet& scr) {
   for (const PlanGroup& G : p.groups)
     k << "|" << G.snapshot << "," << G.method << "," << G.imaging << "," << G.nv << "," << G.nl << "," << G.maxL
       << "," << G.maxnz << "," << G.maxnx << "," << G.maxny << "," << G.total_items << "," << G.tw << "," << G.th
-      << "," << G.bps << "," << G.rscale << "," << G.any_nn << "," << (const void*)G.totpol;
+      << "," << G.bps << "," << G.rscale << "," << G.any_nn << "," << G.item_off[G.bundle_view] << "," << (const void*)G.totpol;
   return k.str();
 }
 

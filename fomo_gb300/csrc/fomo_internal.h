@@ -86,10 +86,11 @@ struct LineDesc {
 // back (segments whose capsule held too many points), their queue head, the
 // number of hard samples queued for a warp each, their queue head, the ray
 // queue head of the emission pass of the two-pass spectral march, the number
-// of records flagged for the far pass and its queue head.
+// of records flagged for the far pass and its queue head, the queue head of the
+// search over 2 x 2 blocks of rays.
 enum MarchCounter {
   kCtrRays = 0, kCtrDeferred, kCtrDeferredHead, kCtrOverflow, kCtrOverflowHead, kCtrHard, kCtrHardHead, kCtrShade,
-  kCtrFar, kCtrFarHead,
+  kCtrFar, kCtrFarHead, kCtrBundles,
   kCtrCount
 };
 
@@ -119,6 +120,9 @@ struct MarchArgs {
   int64_t npos_cap;              // its entries (index checks of the bounds-check build)
   const float* s2;               // Thomson: per-view sin^2(chi) per sorted point (nviews * n), else null
   const float2* totpol;          // Thomson: sorted (n*totterm, n*polterm)
+  const float2* ktf;             // per view and LOS sample: the LOS table's x, -y, z as FP32 pairs (high, low part)
+  int64_t bundle_from;           // work items from here on are searched as 2 x 2 blocks of rays (a multiple of 4)
+  int parts;                     // work units per block of rays: stretches of its segments
   float rscale;                  // gather radius of the search in local point spacings (0: the default, 0.9)
   unsigned long long* stats;     // optional search counters (profiling), else null
   const unsigned* stop;          // a server batch's stop word (device memory), or null: once it is
@@ -207,7 +211,9 @@ cudaError_t launch_speed_max(const float4* vel, int64_t n, unsigned int* vmax_bi
 // view.cu
 cudaError_t launch_view_init(ViewDesc* views, int nviews, cudaStream_t s);
 cudaError_t launch_view_extents(SnapDev snap, ViewDesc* views, int nviews, float* s2, cudaStream_t s);
-cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, int ktab_stride, cudaStream_t s);
+// ktf (null: not wanted) gets the LOS table as FP32 pairs, three per sample.
+cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, float2* ktf, int ktab_stride,
+                                 cudaStream_t s);
 
 // projection.cu: the projection render of every view of a group (outputs zeroed beforehand)
 cudaError_t launch_projection(SnapDev snap, const ViewDesc* views, const LineDesc* lines, int nviews, int nlines,

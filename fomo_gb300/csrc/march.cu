@@ -66,6 +66,8 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fomo_device.cuh"
 #include "fomo_internal.h"
 
@@ -78,6 +80,7 @@ constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
 constexpr int kMinCtas = 4;  // resident CTAs per SM: 16 warps of latency hiding at <= 128 registers
 constexpr int kMinCtasSearch = 7;   // the search-only pass: 28 warps at <= 72 registers (31 KB shared per CTA)
+constexpr int kMinCtasBundle = 5;   // the search over blocks of rays: 20 warps at <= 102 registers (at 64 views x 4 lines: 37.1, 35.4, 38.4, 37.7 ms at 4 to 7 CTAs)
 constexpr int kMinCtasShade = 8;   // the emission-only pass: 32 warps at <= 64 registers
 constexpr int kMinCtasImaging = 5; // imaging / Thomson first pass: 20 warps at <= 102 registers
 constexpr int kMinCtasDeferred = 8; // one-lane ring walks wait on dependent loads: 32 warps (64 registers, some spill)
@@ -163,6 +166,12 @@ __device__ __forceinline__ float warp_min(float v) {
   return v;
 }
 
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
+  return v;
+}
+
 __device__ __forceinline__ int warp_incl_scan(int v) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -207,6 +216,21 @@ __device__ __forceinline__ int find_view(const int64_t* off, int nviews, int64_t
   return lo;
 }
 
+// Pixel (row i, column j) of item `within` of a tw x th ray tile.  Where both
+// sides are even, four consecutive items are a 2 x 2 block of pixels, which
+// march_search_bundle takes together.
+__device__ __forceinline__ void tile_pixel(int within, int tw, int th, int& i, int& j) {
+  if ((tw | th) & 1) {
+    i = within / tw;
+    j = within - i * tw;
+    return;
+  }
+  const int quad = within >> 2, hw = tw >> 1;
+  const int qi = quad / hw;
+  i = 2 * qi + ((within >> 1) & 1);
+  j = 2 * (quad - qi * hw) + (within & 1);
+}
+
 // The ray of work item `item` (views' rays in tile order); false for the
 // padding items of partial tiles.
 __device__ __forceinline__ bool ray_of_item(const MarchArgs& a, const double3* ktab, int ktab_stride,
@@ -218,8 +242,10 @@ __device__ __forceinline__ bool ray_of_item(const MarchArgs& a, const double3* k
   const int tiles_x = (nx + tw - 1) / tw;
   const int tile = local / (tw * th);
   const int within = local - tile * (tw * th);
-  const int i = (tile / tiles_x) * th + within / tw;
-  const int j = (tile % tiles_x) * tw + within % tw;
+  int ti, tj;  // pixel within the tile
+  tile_pixel(within, tw, th, ti, tj);
+  const int i = (tile / tiles_x) * th + ti;
+  const int j = (tile % tiles_x) * tw + tj;
   if (i >= ny || j >= nx) return false;
   // ray position in the image plane (nn:152-153, tabulated per view by the
   // finalize kernel) and the per-ray terms of the derotation (nn:165)
@@ -241,9 +267,9 @@ __device__ __forceinline__ bool ray_of_item(const MarchArgs& a, const double3* k
 }
 
 // Warp-collective: the next ray of the work queue (items item_base ..
-// total_items - 1, head counter `ctr`), false when the queue is drained.
-__device__ __forceinline__ bool next_ray(const MarchArgs& a, const double3* ktab, int ktab_stride, RayCtx& r,
-                                         int ctr = kCtrRays) {
+// end - 1, head counter `ctr`), false when the queue is drained.
+__device__ __forceinline__ bool next_ray(const MarchArgs& a, const double3* ktab, int ktab_stride, int64_t end,
+                                         RayCtx& r, int ctr = kCtrRays) {
   const int lane = threadIdx.x & 31;
   for (;;) {
     unsigned long long item = 0;
@@ -253,10 +279,10 @@ __device__ __forceinline__ bool next_ray(const MarchArgs& a, const double3* ktab
       // drained.  The word only goes from 0 to 1 while a batch runs, so a
       // kernel that starts after one that stopped stops at its first ray too
       // (an emission pass reads no position its search did not write).
-      if (a.stop && __ldcv(a.stop) != 0u) item = (unsigned long long)a.total_items;
+      if (a.stop && __ldcv(a.stop) != 0u) item = (unsigned long long)end;
     }
     item = __shfl_sync(kFull, item, 0) + (unsigned long long)a.item_base;
-    if ((int64_t)item >= a.total_items) return false;
+    if ((int64_t)item >= end) return false;
     if (ray_of_item(a, ktab, ktab_stride, (int64_t)item, r)) return true;
   }
 }
@@ -331,8 +357,8 @@ __device__ __forceinline__ void clip_interval(float a, float d, float inv_d, flo
 // coordinates at most amax), plus a few ulp of the coordinates.  With that
 // margin in the cap, a box smaller than the spacing lies inside the gathered
 // ball whole and an empty one is accepted by the search instead of deferred.
-__device__ __forceinline__ float gather_radius(const MarchArgs& a, const RayCtx& r, float aloc, float amax) {
-  const float md_seg = r.mdf + (amax + r.mdf) * 4.8e-7f + r.mdf * 1.2e-7f;
+__device__ __forceinline__ float gather_radius(const MarchArgs& a, float mdf, float aloc, float amax) {
+  const float md_seg = mdf + (amax + mdf) * 4.8e-7f + mdf * 1.2e-7f;
   const float cap = fmaf(md_seg * 1.7321f, 1.0001f, amax * 4.8e-7f) * 1.0001f;
   return fminf(cap, (a.rscale > 0.0f ? a.rscale : kRScaleDefault) * aloc);
 }
@@ -363,6 +389,11 @@ __device__ __forceinline__ PartOut segment_parts(const MarchArgs& a, const RayCt
   bool need0 = false, need1 = false;
   for (int cur = 0; cur < nseg;) {
     const int pn = min(size, nseg - cur);  // this part: samples s0 + cur .. s0 + cur + pn - 1
+    const int j0 = lane - cur, j1 = lane + 32 - cur;
+    if (!__any_sync(kFull, (act[0] && j0 >= 0 && j0 < pn) || (act[1] && j1 >= 0 && j1 < pn))) {
+      cur += pn;  // none of its samples is open
+      continue;
+    }
     // the part's segment through its first and last targets
     const int la = cur & 31, lb = (cur + pn - 1) & 31;
     const bool ha = cur >= 32, hb = cur + pn - 1 >= 32;
@@ -393,7 +424,7 @@ __device__ __forceinline__ PartOut segment_parts(const MarchArgs& a, const RayCt
     const float aloc = g.h * spacing_cells(mocc);
     const float amax =
         fmaxf(fmaxf(fmaxf(fabsf(ax), fabsf(bx)), fmaxf(fabsf(ay), fabsf(by))), fmaxf(fabsf(az), fabsf(bz)));
-    const float R = gather_radius(a, r, aloc, amax);
+    const float R = gather_radius(a, r.mdf, aloc, amax);
     const float Rg = R * 1.0001f + amax * 2.4e-7f;  // + a few ulp of the coordinates
     const float Rg2 = Rg * Rg * (1.0f + kRelPrune);
     // ---- 1. gather
@@ -671,7 +702,7 @@ __device__ __forceinline__ void segment_search(const MarchArgs& a, const RayCtx&
   const float aloc = g.h * spacing_cells(mocc);
   const float amax =
       fmaxf(fmaxf(fmaxf(fabsf(ax), fabsf(bx)), fmaxf(fabsf(ay), fabsf(by))), fmaxf(fabsf(az), fabsf(bz)));
-  const float R = gather_radius(a, r, aloc, amax);
+  const float R = gather_radius(a, r.mdf, aloc, amax);
   const float Rg = R * 1.0001f + amax * 2.4e-7f;  // + a few ulp of the coordinates
   const float Rg2 = Rg * Rg * (1.0f + kRelPrune);
   // ---- 1. gather
@@ -945,7 +976,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSearch) march_search(MarchAr
   SegSmem& sm = segs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, r)) {
+  while (next_ray(a, ktab, ktab_stride, min(a.total_items, a.bundle_from), r)) {
     const ViewDesc* V = a.views + r.v;
     const int nz = V->nz;
     int32_t* nnout = a.nn_idx ? a.nn_idx[r.v] : nullptr;
@@ -967,6 +998,572 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSearch) march_search(MarchAr
 }
 
 // ---------------------------------------------------------------------------
+// Search pass over 2 x 2 blocks of rays.
+//
+// What bounds the search is instruction issue, and most of it is the gather of
+// a segment's candidates: enumerating its rows of cells, loading their points and
+// testing them against the capsule (61 % of march_search's time, 115 points
+// loaded for 22 kept).  Where pixels are closer than points, neighbouring rays
+// gather almost the same points; here a warp gathers once, around the axis of
+// four rays, for 4 x 64 samples, and each lane then tests every candidate it
+// loads from shared memory against the four rays' samples of its LOS index.
+// 64 views of the 2M-point loop, 256 x 256 x 512: 70.4 ms one ray per warp
+// (28.4 warp instructions per sample, FP64 pipe 36 % busy), 35.4 ms as blocks; one
+// 512^3 view 3.77 -> 1.94 ms; the 8M-point rope, 1024^3, 25.6 -> 12.9 ms.
+//
+//  - A lane's four targets are A_r + z_k, r the ray: A and z as FP32 pairs, added
+//    with a two-sum.  The FP32 target the reference rounds from its FP64 sum
+//    is the rounding of hi + (lo +- E) for both signs of a bound E on what the
+//    pairs drop; where the two differ (a few per million) the lane adds in
+//    FP64.  FP64 runs at 1/64 of the FP32 rate here: three additions and three
+//    conversions per sample were a third of march_search's time.
+//  - Rows are listed in shared memory first (a prefix sum over the non-empty ones),
+//    then their points are loaded in full rounds of 32; the row of a point comes
+//    from a bit mask of the rows that start in the round.
+//  - R is the gather radius of one ray; the capsule's radius is R + e, e the
+//    rays' distance from the axis, so every point within R of every sample is
+//    gathered: a winner nearer than R is final.
+//  - A segment that would hold more than kBunCap candidates is taken in parts
+//    of 32, 16 or 8 samples; where that does not do (points much denser than
+//    pixels), its rays go to march_split one by one.
+// ---------------------------------------------------------------------------
+constexpr int kBunCap = 208;  // candidates per part (sized so that 7 CTAs fit an SM)
+
+struct __align__(16) BundleSmem {
+  // [0, kBunCap): gathered candidates (x, y, z, sorted position); [kBunCap, 2 kBunCap):
+  // the same in sample order, and before that the row list of the gather
+  float4 q[2 * kBunCap];
+  double a[4][3];   // the rays' terms of the derotation (RayCtx::A0, A1, A2)
+  float4 af[4][2];  // the same as FP32 pairs: (A0 high, low, A1 high, low), (A2 high, low, -, -)
+  int bstart[kSeg + 1];
+  int cursor[kSeg];
+  unsigned need[8];  // per ray: samples 0-31 and 32-63 of the segment left open
+  unsigned char cb[kBunCap];
+};
+constexpr int kBunRows = 2 * kBunCap;  // rows the list holds (8 bytes each)
+constexpr int kBunPart = 8;            // samples of the smallest part
+// The part size below pn (> kBunPart): 32, 16 or 8 samples, so that parts do not straddle the mask words.
+__device__ __forceinline__ int smaller_part(int pn) { return pn > 32 ? 32 : pn > 16 ? 16 : 8; }
+
+// Exact re-rank of a near-tie among candidates [c0, c1) (see exact_rerank_list);
+// w holds the sorted position, the original index comes from the points.
+__device__ __noinline__ int exact_rerank_pos(const float4* sq, int c0, int c1, float tx, float ty, float tz,
+                                             float md_in, float band, const float4* pts, int64_t n) {
+  double bestD = DBL_MAX;
+  int bestOrig = 0x7fffffff, bpos = -1;
+  for (int c = c0; c < c1; ++c) {
+    const float4 q = sq[c];
+    const float dx = q.x - tx, dy = q.y - ty, dz = q.z - tz;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    const float cheb = fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz));
+    if (cheb < md_in && d2 <= band) {
+      const double D = exact_dist2(q.x, q.y, q.z, tx, ty, tz);
+      const int p = __float_as_int(q.w);
+      const int o = __float_as_int(__ldg(&pts[FOMO_IDX(p, n, kSitePts)].w));
+      if (D < bestD || (D == bestD && o < bestOrig)) {
+        bestD = D;
+        bestOrig = o;
+        bpos = p;
+      }
+    }
+  }
+  return bpos;
+}
+
+// fl(A + z) for A = ah + al and z = zh + zl up to E: false where E decides.
+__device__ __forceinline__ bool pair_target(float ah, float al, float2 z, float E, float& t) {
+  const float s = __fadd_rn(ah, z.x), bb = __fsub_rn(s, ah);
+  const float e = __fadd_rn(__fadd_rn(__fsub_rn(ah, __fsub_rn(s, bb)), __fsub_rn(z.x, bb)), __fadd_rn(al, z.y));
+  t = __fadd_rn(s, __fadd_rn(e, E));
+  return t == __fadd_rn(s, __fsub_rn(e, E));
+}
+
+// The candidates [c0, c1) against a lane's four targets: per target the nearest
+// (b1, its index bi) and the second best (b2).  BOX: only candidates within
+// md_in of the target on every axis count, and amb gets bit r where one lies
+// within [md_in, md_out] (a few ulp of a box face).  Without BOX every
+// candidate nearer than b1's start value lies inside the box.
+template <bool BOX>
+__device__ __forceinline__ void bundle_scan(const float4* sq, int c0, int c1, const float (&tx)[4], const float (&ty)[4],
+                                            const float (&tz)[4], float md_in, float md_out, float (&b1)[4],
+                                            float (&b2)[4], int (&bi)[4], unsigned& amb) {
+#pragma unroll 1
+  for (int c = c0; c < c1; ++c) {  // four independent targets per load; unrolled further, the code outgrows the instruction cache
+    const float4 q = sq[c];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float dx = q.x - tx[r], dy = q.y - ty[r], dz = q.z - tz[r];
+      float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      if (BOX) {
+        const float cheb = fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz));
+        if (!(cheb < md_in)) {
+          d2 = FLT_MAX;
+          if (cheb <= md_out) amb |= 1u << r;
+        }
+      }
+      b2[r] = fminf(b2[r], fmaxf(b1[r], d2));
+      if (d2 < b1[r]) {
+        b1[r] = d2;
+        bi[r] = c;
+      }
+    }
+  }
+}
+
+// sum of `occ` over the warp as the mean occupancy of a cell, and the local point
+// spacing there
+__device__ __forceinline__ float mean_occupancy(const SnapDev& S, float ax, float ay, float az, float sdx, float sdy,
+                                                float sdz) {
+  const GridParams& g = S.g;
+  const float fs = (float)(threadIdx.x & 31) * (1.0f / 31.0f);
+  const float px = fmaf(fs, sdx, ax), py = fmaf(fs, sdy, ay), pz = fmaf(fs, sdz, az);
+  int occ = 0;
+  if (px >= g.minx && px <= g.maxx && py >= g.miny && py <= g.maxy && pz >= g.minz && pz <= g.maxz) {
+    const int c = (cell_coord(pz, g.oz, g.inv_h, g.dz) * g.dy + cell_coord(py, g.oy, g.inv_h, g.dy)) * g.dx +
+                  cell_coord(px, g.ox, g.inv_h, g.dx);
+    occ = __ldg(S.cell_start + FOMO_IDX(c + 1, cell_entries(g), kSiteCellStart)) -
+          __ldg(S.cell_start + FOMO_IDX(c, cell_entries(g), kSiteCellStart));
+  }
+  return fmaxf((float)__reduce_add_sync(kFull, (unsigned)occ) * (1.0f / 32.0f), 0.125f);
+}
+
+// Warp-collective: the points of rows [0, nlist) of the row list, those within Rg
+// of the axis a + s d appended to sm.q from `count` on with the bucket they
+// project on (pn samples).  total: points in the listed rows.
+__device__ __forceinline__ void gather_rows(const SnapDev& S, BundleSmem& sm, const int2* rows, int nlist, int total,
+                                            float ax, float ay, float az, float sdx, float sdy, float sdz,
+                                            float inv_len2, float Rg2, int pn, int& count) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  int rp = 0;  // the row that holds point ib
+  for (int ib = 0; ib < total; ib += 32) {
+    // rows (each at least one point long) that start in (ib, ib + 32)
+    const int st = rp + 1 + lane < nlist ? rows[rp + 1 + lane].x - ib : 32;
+    const unsigned starts = __reduce_or_sync(kFull, st < 32 ? 1u << st : 0u);
+    const int own = rp + __popc(starts & (lt | (1u << lane)));
+    rp += __popc(starts);
+    const int i = ib + lane;
+    bool keep = false;
+    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+    int bk = 0;
+    if (i < total) {
+      const int p = i + rows[FOMO_IDX(own, kBunRows, kSiteSmem)].y;
+      q = __ldg(S.pts + FOMO_IDX(p, S.n, kSitePts));
+      q.w = __int_as_float(p);
+      const float wx = q.x - ax, wy = q.y - ay, wz = q.z - az;
+      float s = fmaf(wz, sdz, fmaf(wy, sdy, wx * sdx)) * inv_len2;
+      s = fminf(fmaxf(s, 0.0f), 1.0f);
+      const float ex = fmaf(-s, sdx, wx), ey = fmaf(-s, sdy, wy), ez = fmaf(-s, sdz, wz);
+      keep = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= Rg2;
+      bk = min(max(__float2int_rn(s * (float)(pn - 1)), 0), pn - 1);
+    }
+    // the next row may start at the next round's first point
+    if (rp + 1 < nlist && rows[rp + 1].x == ib + 32) ++rp;
+    const unsigned msk = __ballot_sync(kFull, keep);
+    if (keep) {
+      const int slot = count + __popc(msk & lt);
+      if (slot < kBunCap) {
+        sm.q[slot] = q;
+        sm.cb[slot] = (unsigned char)bk;
+      }
+    }
+    count += __popc(msk);
+    if (count > kBunCap) return;  // the part is taken again in smaller ones
+  }
+}
+
+template <bool STATS>
+__global__ void __launch_bounds__(kThreads, kMinCtasBundle)
+    march_search_bundle(MarchArgs a, const double3* __restrict__ ktab, int ktab_stride) {
+  __shared__ BundleSmem segs[kWarps];
+  BundleSmem& sm = segs[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const SnapDev& S = a.snap;
+  const GridParams& g = S.g;
+  for (;;) {
+    // the next unit: one of a.parts stretches of a bundle's segments
+    unsigned long long unit = 0;
+    if (lane == 0) {
+      unit = atomicAdd(a.counter + kCtrBundles, 1ull);
+      if (a.stop && __ldcv(a.stop) != 0u) unit = (unsigned long long)a.total_items * (unsigned)a.parts;  // see next_ray
+    }
+    unit = __shfl_sync(kFull, unit, 0);
+    const int64_t bundle = (int64_t)(unit / (unsigned)a.parts);
+    const int part = (int)(unit - (unsigned long long)bundle * (unsigned)a.parts);
+    const int64_t item = max(a.item_base, a.bundle_from) + 4 * bundle;
+    if (item >= a.total_items) return;
+    const int v = find_view(a.ray_offset, a.nviews, item);
+    const ViewDesc* V = a.views + v;
+    const int nx = V->nx, ny = V->ny, nz = V->nz;
+    int i0, j0;
+    {
+      const int tw = V->ray_tile_w, th = V->ray_tile_h;
+      const int local = (int)(item - __ldg(a.ray_offset + v));
+      const int tiles_x = (nx + tw - 1) / tw;
+      const int tile = local / (tw * th);
+      int ti, tj;
+      tile_pixel(local - tile * (tw * th), tw, th, ti, tj);
+      i0 = (tile / tiles_x) * th + ti;
+      j0 = (tile % tiles_x) * tw + tj;
+    }
+    const int nsegs = (nz + kSeg - 1) / kSeg;
+    const int seg0 = (int)((int64_t)nsegs * part / a.parts), seg1 = (int)((int64_t)nsegs * (part + 1) / a.parts);
+    if (i0 >= ny || j0 >= nx || seg0 >= seg1) continue;  // a tile's padding, or a view with fewer segments
+    const unsigned valid = (1u | (j0 + 1 < nx ? 2u : 0u)) * (1u | (i0 + 1 < ny ? 4u : 0u));  // bit r: ray r is in the image
+    const double3* kt = ktab + (int64_t)v * ktab_stride;
+    const float2* ktf = a.ktf + 3 * (int64_t)v * ktab_stride;
+    const float mdf = __double2float_rn(V->md);
+    int32_t* nnout = a.nn_idx ? a.nn_idx[v] : nullptr;
+    // the rays' terms of the derotation (nn:165; ray r of the bundle in lanes r, r + 4, ..; a ray
+    // outside the image stands on its neighbour), their axis and distance from it
+    float cx, cy, cz, e, E;
+    {
+      const double x = V->xt[FOMO_IDX(min(j0 + (lane & 1), nx - 1), nx, kSiteRayXY)];
+      const double y = V->yt[FOMO_IDX(min(i0 + ((lane >> 1) & 1), ny - 1), ny, kSiteRayXY)];
+      const double cb = V->cb, sb = V->sb, cl = V->cl, sl = V->sl;
+      double A[3];
+      A[0] = __dadd_rn(__dmul_rn(__dmul_rn(x, cb), cl), __dmul_rn(y, sl));
+      A[1] = __dadd_rn(__dmul_rn(__dmul_rn(-x, cb), sl), __dmul_rn(y, cl));
+      A[2] = __dmul_rn(-x, sb);
+      float f[3], lo[3], c[3], big = 0.0f, d2 = 0.0f;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        f[d] = __double2float_rn(A[d]);
+        lo[d] = __double2float_rn(__dsub_rn(A[d], (double)f[d]));
+        if (lane < 4) sm.a[lane][d] = A[d];
+        c[d] = f[d] + __shfl_xor_sync(kFull, f[d], 1);
+        c[d] = 0.25f * (c[d] + __shfl_xor_sync(kFull, c[d], 2));
+        c[d] = __shfl_sync(kFull, c[d], 0);
+        big = fmaxf(big, fabsf(f[d]));
+        d2 = fmaf(f[d] - c[d], f[d] - c[d], d2);
+      }
+      if (lane < 4) {
+        sm.af[lane][0] = make_float4(f[0], lo[0], f[1], lo[1]);
+        sm.af[lane][1] = make_float4(f[2], lo[2], 0.0f, 0.0f);
+      }
+      big = warp_max(big);
+      e = sqrtf(warp_max(d2));
+      cx = c[0];
+      cy = c[1];
+      cz = c[2];
+      // the LOS table is linear in the sample, so its ends bound it
+      const float2 *z0 = ktf, *z1 = ktf + 3 * (nz - 1);
+      float zbig = 0.0f;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) zbig = fmaxf(zbig, fmaxf(fabsf(z0[d].x), fabsf(z1[d].x)));
+      E = (big + zbig) * 5.7e-14f;  // 2^-44: twice what the pairs and their sums can drop
+    }
+    __syncwarp();
+    for (int s0 = seg0 * kSeg; s0 < min(seg1 * kSeg, nz); s0 += kSeg) {
+      const int nseg = min(kSeg, nz - s0);
+      if (lane < 8) sm.need[lane] = 0u;
+      bool over = false;
+      int size = kSeg;
+      int st_rows = 0, st_loaded = 0, st_cand = 0, st_split = 0;
+      unsigned st_scanned = 0, st_ties = 0, st_amb = 0, st_nocand = 0, st_far = 0;
+      for (int cur = 0; cur < nseg;) {
+        const int pn = min(size, nseg - cur);  // this part: samples s0 + cur .. s0 + cur + pn - 1
+        // its stretch of the axis
+        const float2 *z0 = ktf + 3 * (s0 + cur), *z1 = z0 + 3 * (pn - 1);
+        const float ax = cx + z0[0].x, ay = cy + z0[1].x, az = cz + z0[2].x;
+        const float bx = cx + z1[0].x, by = cy + z1[1].x, bz = cz + z1[2].x;
+        const float sdx = bx - ax, sdy = by - ay, sdz = bz - az;
+        const float len2 = fmaf(sdz, sdz, fmaf(sdy, sdy, sdx * sdx));
+        const float inv_len2 = len2 > 0.0f ? 1.0f / len2 : 0.0f;
+        const float len = sqrtf(len2);
+        const float mocc = mean_occupancy(S, ax, ay, az, sdx, sdy, sdz);
+        const float amax =
+            e + fmaxf(fmaxf(fmaxf(fabsf(ax), fabsf(bx)), fmaxf(fabsf(ay), fabsf(by))),
+                      fmaxf(fmaxf(fabsf(az), fabsf(bz)), fmaxf(fmaxf(fabsf(cx), fabsf(cy)), fabsf(cz))));
+        const float R = gather_radius(a, mdf, g.h * spacing_cells(mocc), amax);
+        // a sample lies within e of the axis, up to the rounding of its target, the axis and
+        // the points' distances (a few ulp of the coordinates)
+        const float Rg = (R + e) * 1.0001f + amax * 9.6e-7f;
+        const float Rg2 = Rg * Rg * (1.0f + kRelPrune);
+        // the candidates to expect: parts of fewer samples where a whole segment would not fit, no
+        // gather where the smallest would not.  With the rays farther from the axis than R the
+        // capsule holds over four times one ray's points, and parts below 32 samples cost more than
+        // march_split's of one ray (0.5M-point rope, 256^2 x 256: search 918 against 595 us)
+        const float per_len = mocc * g.inv_h * g.inv_h * g.inv_h * 3.1416f * Rg * Rg;
+        const int least = e <= R ? kBunPart : 32;
+        const bool parts_fit = per_len * (len * ((float)least / (float)pn) + 1.33f * Rg) < 1.1f * kBunCap;
+        bool gathered = parts_fit || pn <= least;
+        if (gathered && pn > least && per_len * (len + 1.33f * Rg) > 1.1f * kBunCap) {
+          size = smaller_part(pn);
+          continue;
+        }
+        // ---- 1. gather
+        int count = 0;
+        const float cxl = fmaxf(fminf(ax, bx) - Rg, g.minx), cxh = fminf(fmaxf(ax, bx) + Rg, g.maxx);
+        const float cyl = fmaxf(fminf(ay, by) - Rg, g.miny), cyh = fminf(fmaxf(ay, by) + Rg, g.maxy);
+        const float czl = fmaxf(fminf(az, bz) - Rg, g.minz), czh = fminf(fmaxf(az, bz) + Rg, g.maxz);
+        if (gathered && cxl <= cxh && cyl <= cyh && czl <= czh) {
+          const int x0 = cell_coord(cxl, g.ox, g.inv_h, g.dx), x1 = cell_coord(cxh, g.ox, g.inv_h, g.dx);
+          const int y0 = cell_coord(cyl, g.oy, g.inv_h, g.dy), y1 = cell_coord(cyh, g.oy, g.inv_h, g.dy);
+          const int k0 = cell_coord(czl, g.oz, g.inv_h, g.dz), k1 = cell_coord(czh, g.oz, g.inv_h, g.dz);
+          const int nyr = y1 - y0 + 1, nzr = k1 - k0 + 1;
+          const int nrows = nyr * nzr;
+          st_rows += nrows;
+          if (nrows > kMaxRows) {
+            gathered = false;
+          } else {
+            int2* const rows = reinterpret_cast<int2*>(sm.q + kBunCap);  // (first point's number, position - number)
+            const float m = kCellMargin * g.h;
+            const float mR = m + Rg, xm = Rg + m + 2e-4f * len;
+            // (an axis along a slab: its clip is all or nothing)
+            const float inv_dy = fabsf(sdy) > 1e-30f ? 1.0f / sdy : 1e30f;
+            const float inv_dz = fabsf(sdz) > 1e-30f ? 1.0f / sdz : 1e30f;
+            const float inv_nyr = 1.0f / (float)nyr;
+            int nlist = 0, total = 0;
+            for (int rb = 0; rb < nrows && count <= kBunCap; rb += 32) {
+              const int rr = rb + lane;
+              int n = 0, base = 0;
+              if (rr < nrows) {
+                int ry;
+                const int rz = row_div(rr, nyr, inv_nyr, ry);
+                const int jy = y0 + ry, kz = k0 + rz;
+                // the stretch [slo, shi] of the axis within Rg of the row's slabs
+                const float ty1 = (fmaf((float)jy, g.h, g.oy) - mR - ay) * inv_dy,
+                            ty2 = (fmaf((float)(jy + 1), g.h, g.oy) + mR - ay) * inv_dy;
+                const float tz1 = (fmaf((float)kz, g.h, g.oz) - mR - az) * inv_dz,
+                            tz2 = (fmaf((float)(kz + 1), g.h, g.oz) + mR - az) * inv_dz;
+                const float slo = fmaxf(fmaxf(fminf(ty1, ty2), fminf(tz1, tz2)) - 1e-4f, 0.0f);
+                const float shi = fminf(fminf(fmaxf(ty1, ty2), fmaxf(tz1, tz2)) + 1e-4f, 1.0f);
+                if (slo <= shi) {
+                  const float xa = fmaf(slo, sdx, ax), xb = fmaf(shi, sdx, ax);
+                  const int c0 = max(x0, cell_coord(fminf(xa, xb) - xm, g.ox, g.inv_h, g.dx));
+                  const int c1 = min(x1, cell_coord(fmaxf(xa, xb) + xm, g.ox, g.inv_h, g.dx));
+                  if (c0 <= c1) {
+                    const int rowbase = (kz * g.dy + jy) * g.dx;
+                    base = __ldg(S.cell_start + FOMO_IDX(rowbase + c0, cell_entries(g), kSiteCellStart));
+                    n = __ldg(S.cell_start + FOMO_IDX(rowbase + c1 + 1, cell_entries(g), kSiteCellStart)) - base;
+                  }
+                }
+              }
+              const int incl = warp_incl_scan(n);
+              const unsigned ne = __ballot_sync(kFull, n > 0);
+              if (n > 0) {
+                const int first = total + incl - n;
+                rows[FOMO_IDX(nlist + __popc(ne & ((1u << lane) - 1u)), kBunRows, kSiteSmem)] = make_int2(first, base - first);
+              }
+              nlist += __popc(ne);
+              total += __shfl_sync(kFull, incl, 31);
+              if (nlist > kBunRows - 32 || rb + 32 >= nrows) {  // the list is full, or complete
+                __syncwarp();
+                gather_rows(S, sm, rows, nlist, total, ax, ay, az, sdx, sdy, sdz, inv_len2, Rg2, pn, count);
+                st_loaded += total;
+                nlist = 0;
+                total = 0;
+                __syncwarp();
+              }
+            }
+            if (count > kBunCap) gathered = false;
+          }
+        }
+        if (!gathered && pn > least) {
+          ++st_split;
+          if (parts_fit) {
+            size = smaller_part(pn);  // the same samples again in smaller parts
+            continue;
+          }
+        }
+        const int ncand = gathered ? count : 0;
+        st_cand += ncand;
+        // ---- 2. counting sort by sample index
+        sm.cursor[lane] = 0;
+        sm.cursor[lane + 32] = 0;
+        __syncwarp();
+        for (int c = lane; c < ncand; c += 32) atomicAdd(&sm.cursor[FOMO_IDX(sm.cb[c], kSeg, kSiteSmem)], 1);
+        __syncwarp();
+        {
+          const int h0 = sm.cursor[2 * lane], h1 = sm.cursor[2 * lane + 1];
+          const int incl = warp_incl_scan(h0 + h1);
+          const int ex = incl - h0 - h1;
+          __syncwarp();
+          sm.bstart[2 * lane] = ex;
+          sm.bstart[2 * lane + 1] = ex + h0;
+          if (lane == 31) sm.bstart[kSeg] = incl;
+          sm.cursor[2 * lane] = ex;
+          sm.cursor[2 * lane + 1] = ex + h0;
+        }
+        __syncwarp();
+        for (int c = lane; c < ncand; c += 32)
+          sm.q[kBunCap + FOMO_IDX(atomicAdd(&sm.cursor[FOMO_IDX(sm.cb[c], kSeg, kSiteSmem)], 1), kBunCap, kSiteSmem)] = sm.q[c];
+        __syncwarp();
+        const float4* sq = sm.q + kBunCap;  // the candidates in sample order
+        // ---- 3./4. scan of the buckets within R, acceptance
+        const float dlt = (pn > 1) ? len / (float)(pn - 1) : 0.0f;
+        // buckets that can hold a candidate within R of a sample (half a bucket and the targets' rounding on top)
+        const int w = (dlt > 0.0f) ? (int)fminf((R * 1.0001f + amax * 1e-6f) / dlt + 0.51f, (float)kSeg) : kSeg;
+        const float R2 = R * R * (1.0f - 2.0f * kRelPrune);
+        const float delta = (amax + mdf) * 4.8e-7f + mdf * 1.2e-7f;  // ~4 ulp of the box corners
+        const float md_in = mdf - delta, md_out = mdf + delta;
+        const bool box = R >= md_in;                              // a winner may lie outside its box
+        const bool whole = md_out * 1.7321f * 1.0001f < R;        // a sample's box lies in its gathered ball
+        // some sample's box may miss the points' bounding box
+        const float er = e + amax * 1e-6f - md_out;
+        const bool edge = fminf(ax, bx) - er <= g.minx || fmaxf(ax, bx) + er >= g.maxx || fminf(ay, by) - er <= g.miny ||
+                          fmaxf(ay, by) + er >= g.maxy || fminf(az, bz) - er <= g.minz || fmaxf(az, bz) + er >= g.maxz;
+#pragma unroll 1
+        for (int jb = 0; jb < pn; jb += 32) {
+          const int j = jb + lane;
+          const bool act = j < pn;
+          const int k = min(s0 + cur + j, nz - 1);
+          float tx[4], ty[4], tz[4];
+          {
+            const float2* zk = ktf + 3 * (int64_t)FOMO_IDX(k, nz, kSiteKtab);
+            const float2 zx = __ldg(zk), zy = __ldg(zk + 1), zz = __ldg(zk + 2);
+            bool ok = true;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const float4 xy = sm.af[r][0], z = sm.af[r][1];
+              ok = pair_target(xy.x, xy.y, zx, E, tx[r]) && ok;
+              ok = pair_target(xy.z, xy.w, zy, E, ty[r]) && ok;
+              ok = pair_target(z.x, z.y, zz, E, tz[r]) && ok;
+            }
+            if (__builtin_expect(!ok, 0)) {
+              const double3 zd = kt[k];
+#pragma unroll
+              for (int r = 0; r < 4; ++r) {
+                tx[r] = __double2float_rn(__dadd_rn(sm.a[r][0], zd.x));
+                ty[r] = __double2float_rn(__dsub_rn(sm.a[r][1], zd.y));
+                tz[r] = __double2float_rn(__dadd_rn(sm.a[r][2], zd.z));
+              }
+            }
+          }
+          float b1[4], b2[4];
+          int bi[4];
+          unsigned amb = 0;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            b1[r] = R2;  // farther candidates cannot be accepted
+            b2[r] = FLT_MAX;
+            bi[r] = -1;
+          }
+          const int c0 = sm.bstart[max(j - w, 0)], c1 = act ? sm.bstart[min(j + w, pn - 1) + 1] : c0;
+          if (gathered) {
+            if (box)
+              bundle_scan<true>(sq, c0, c1, tx, ty, tz, md_in, md_out, b1, b2, bi, amb);
+            else
+              bundle_scan<false>(sq, c0, c1, tx, ty, tz, md_in, md_out, b1, b2, bi, amb);
+          }
+          // a sample is settled with a candidate, or when its box holds no point: it lies in the
+          // gathered ball, or outside the points' bounding box (hi <= min or lo >= max on some axis)
+          unsigned done = gathered && whole ? 15u : 0u, tie = 0u;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            if (bi[r] >= 0) done |= 1u << r;
+            if (b2[r] <= b1[r] * (1.0f + kRelTie)) tie |= 1u << r;
+          }
+          if (edge && gathered) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              if ((tx[r] + md_out <= g.minx) || (tx[r] - md_out >= g.maxx) || (ty[r] + md_out <= g.miny) ||
+                  (ty[r] - md_out >= g.maxy) || (tz[r] + md_out <= g.minz) || (tz[r] - md_out >= g.maxz))
+                done |= 1u << r;
+          }
+          done &= ~amb;
+          int pres[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            pres[r] = (done >> r) & 1u && bi[r] >= 0 ? __float_as_int(sq[FOMO_IDX(bi[r], kBunCap, kSiteSmem)].w) : -1;
+          if (__builtin_expect((tie & done) != 0u, 0)) {
+            // possible FP64 ties: exact re-rank of the in-box contenders
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              if ((tie & done) >> r & 1u && bi[r] >= 0)
+                pres[r] = exact_rerank_pos(sq, c0, c1, tx[r], ty[r], tz[r], md_in, b1[r] * (1.0f + kRelTie), S.pts, S.n);
+          }
+          int32_t* row = a.npos + (item - a.item_base) * ktab_stride + k;
+#pragma unroll
+          for (int r = 0; r < 4; ++r, row += ktab_stride) {
+            const bool on = (valid >> r) & 1u;
+            if (on && act) __stcs(a.npos + FOMO_IDX(row - a.npos, a.npos_cap, kSiteNpos), pres[r]);
+            const unsigned need = __ballot_sync(kFull, on && act && !((done >> r) & 1u));
+            if (need && lane == 0) sm.need[2 * r + ((cur + jb) >> 5)] |= need << ((cur + jb) & 31);
+          }
+          if (nnout && act) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+              if ((valid >> r) & 1u)
+                nnout[FOMO_IDX(((int64_t)(i0 + (r >> 1)) * nx + j0 + (r & 1)) * nz + k, (int64_t)nx * ny * nz, kSiteNnIdx)] =
+                    pres[r] >= 0 ? __float_as_int(S.pts[FOMO_IDX(pres[r], S.n, kSitePts)].w) : -1;
+          }
+          if (STATS && act) {
+            st_scanned += (unsigned)(c1 - c0);
+            st_ties += __popc(tie & done & valid);
+            st_amb += __popc(amb & valid);
+            if (gathered) (ncand ? st_far : st_nocand) += __popc(~(done | amb) & valid);
+          }
+        }
+        if (!gathered) over = true;
+        __syncwarp();  // the candidate lists are rewritten by the next part
+        cur += pn;
+      }
+      // ---- 5. samples left open: one record per ray, as march_search writes them
+      if (lane < 4) {
+        const unsigned f0 = sm.need[2 * lane], f1 = sm.need[2 * lane + 1];
+        if (f0 | f1) {
+          const unsigned long long q = atomicAdd(a.counter + (over ? kCtrOverflow : kCtrDeferred), 1ull);
+          const int64_t slot = over ? a.deferred_cap - 1 - (int64_t)q : (int64_t)q;
+          unsigned flags = 0u;
+          if (a.far_list && mdf >= kFarBox * g.h) {
+            // the halves the far pass may take (see segment_search), by the bundle's axis
+            const float off2 = kFarOut2 * g.h * g.h;
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+              if (__popc(hh ? f1 : f0) < kFarMin) continue;
+              const float2 *z0 = ktf + 3 * (s0 + min(32 * hh, nseg - 1)), *z1 = ktf + 3 * (s0 + min(32 * hh + 31, nseg - 1));
+              const float xa = cx + z0[0].x, xb = cx + z1[0].x, ya = cy + z0[1].x, yb = cy + z1[1].x, za = cz + z0[2].x,
+                          zb = cz + z1[2].x;
+              const float ex = fmaxf(fmaxf(g.minx - fmaxf(xa, xb), fminf(xa, xb) - g.maxx), 0.0f);
+              const float ey = fmaxf(fmaxf(g.miny - fmaxf(ya, yb), fminf(ya, yb) - g.maxy), 0.0f);
+              const float ez = fmaxf(fmaxf(g.minz - fmaxf(za, zb), fminf(za, zb) - g.maxz), 0.0f);
+              if (fmaf(ez, ez, fmaf(ey, ey, ex * ex)) >= off2) flags |= hh ? kRecFar1 : kRecFar0;
+            }
+          }
+          if (slot >= 0 && slot < a.deferred_cap) {  // always: the capacity is one record per segment
+            a.deferred[FOMO_IDX(slot, a.deferred_cap, kSiteDeferred)] = make_uint4((unsigned)item + lane, (unsigned)s0 | flags, f0, f1);
+            if (flags) {
+              const unsigned long long f = atomicAdd(a.counter + kCtrFar, 1ull);
+              if ((int64_t)f < a.deferred_cap) a.far_list[FOMO_IDX(f, a.deferred_cap, kSiteDeferred)] = (int32_t)slot;
+            }
+          }
+        }
+      }
+      if (STATS) {
+        unsigned long long* const stats = a.stats;
+        const int nval = __popc(valid);
+        unsigned open = lane < 8 ? __popc(sm.need[lane]) : 0u;
+        unsigned recs = lane < 4 && (sm.need[2 * lane] | sm.need[2 * lane + 1]) ? 1u : 0u;
+        open = __reduce_add_sync(kFull, open);
+        recs = __reduce_add_sync(kFull, recs);
+        const unsigned sc = __reduce_add_sync(kFull, st_scanned), ti = __reduce_add_sync(kFull, st_ties);
+        const unsigned am = __reduce_add_sync(kFull, st_amb), nc = __reduce_add_sync(kFull, st_nocand),
+                       fa = __reduce_add_sync(kFull, st_far);
+        if (lane == 0) {
+          atomicAdd(stats + kStatSegments, (unsigned long long)nval);
+          atomicAdd(stats + kStatCandidates, (unsigned long long)st_cand);
+          atomicAdd(stats + kStatRows, (unsigned long long)st_rows);
+          atomicAdd(stats + kStatPointsLoaded, (unsigned long long)st_loaded);
+          atomicAdd(stats + kStatNotGathered, (unsigned long long)(st_split + (over ? nval : 0)));
+          atomicAdd(stats + kStatFallbacks, (unsigned long long)open);
+          atomicAdd(stats + kStatDeferredRecs, (unsigned long long)recs);
+          atomicAdd(stats + kStatSamples, (unsigned long long)(nval * nseg));
+          atomicAdd(stats + kStatScanned, 4ull * sc);
+          atomicAdd(stats + kStatTies, (unsigned long long)ti);
+          atomicAdd(stats + kStatFbAmb, (unsigned long long)am);
+          atomicAdd(stats + kStatFbNoCand, (unsigned long long)nc);
+          atomicAdd(stats + kStatFbFar, (unsigned long long)fa);
+        }
+      }
+      __syncwarp();  // need is cleared by the next segment
+    }
+    __syncwarp();  // the rays' terms are rewritten by the next unit
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Spectroscopic march: NL lines x up to NB 32-bin windows per line; lane
 // `lane` owns bins wstart + 32 m + lane of each line.
 // ---------------------------------------------------------------------------
@@ -981,7 +1578,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtas)
   SegSmem& sm = segs[w];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, r)) {
+  while (next_ray(a, ktab, ktab_stride, a.total_items, r)) {
     const ViewDesc* V = a.views + r.v;
     const int nz = V->nz, L = V->L, nx = V->nx;
     const float ux = V->ux, uy = V->uy, uz = V->uz;
@@ -1117,7 +1714,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasImaging)
   SegSmem& sm = segs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, r)) {
+  while (next_ray(a, ktab, ktab_stride, a.total_items, r)) {
     const ViewDesc* V = a.views + r.v;
     const int nz = V->nz, nx = V->nx;
     const LineDesc* LD = a.lines + (int64_t)r.v * a.nlines;
@@ -1262,7 +1859,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasShade)
   const int group = lane >> 3;
   RayCtx r;
   int view = -1;
-  while (next_ray(a, ktab, ktab_stride, r, kCtrShade)) {
+  while (next_ray(a, ktab, ktab_stride, a.total_items, r, kCtrShade)) {
     const ViewDesc* V = a.views + r.v;
     const int L = V->L, nx = V->nx;
     const float ux = V->ux, uy = V->uy, uz = V->uz;
@@ -1380,7 +1977,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasShade)
   __shared__ RunRing rings[kWarps];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, r, kCtrShade)) {
+  while (next_ray(a, ktab, ktab_stride, a.total_items, r, kCtrShade)) {
     const ViewDesc* V = a.views + r.v;
     const LineDesc* LD = a.lines + (int64_t)r.v * a.nlines;
     float acc[NL], comp[NL];
@@ -2023,12 +2620,6 @@ __device__ __forceinline__ int ford(float f) {
 }
 __device__ __forceinline__ float fdeord(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(kFull, v, o));
-  return v;
-}
-
 // Warp-collective search of the lanes' samples (act: this lane holds one, box
 // q).  Returns the lanes whose neighbour was found: pos / orig set, -1 when
 // the box holds no point.
@@ -2428,16 +3019,17 @@ __global__ void __launch_bounds__(kThreads, kMinCtas) march_hard(MarchArgs a, co
   }
 }
 
+// units: work units of the kernel's queue, one per warp (-1: the launch's work items).
 template <typename K>
 cudaError_t launch_persistent(K kernel, const MarchArgs& a, const double3* ktab, int ktab_stride, int sm_count,
-                              cudaStream_t s, int blocks_per_sm_hint) {
+                              cudaStream_t s, int blocks_per_sm_hint, int64_t units = -1) {
   int per_sm = 0;
   cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) per_sm = 1;
   if (blocks_per_sm_hint > 0 && blocks_per_sm_hint < per_sm) per_sm = blocks_per_sm_hint;
   int64_t blocks = (int64_t)sm_count * per_sm;
-  const int64_t cap = (a.total_items - a.item_base + kWarps - 1) / kWarps;
+  const int64_t cap = ((units < 0 ? a.total_items - a.item_base : units) + kWarps - 1) / kWarps;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   kernel<<<(unsigned)blocks, kThreads, 0, s>>>(a, ktab, ktab_stride);
@@ -2543,7 +3135,19 @@ cudaError_t launch_march(const MarchArgs& a, const double3* ktab, int ktab_strid
   mark(-1);
   cudaError_t e;
   if (a.npos) {
-    e = launch_persistent(march_search, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint);
+    e = cudaSuccess;
+    const int64_t single = std::min(a.total_items, a.bundle_from) - a.item_base;
+    const int64_t bundles = (a.total_items - std::max(a.item_base, a.bundle_from)) / 4;
+    if (single > 0) e = launch_persistent(march_search, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint, single);
+    if (e == cudaSuccess && bundles > 0) {
+      // a unit is a stretch of a bundle's segments: all of them where there are
+      // bundles enough for four units per warp of the GPU, single segments at the least
+      MarchArgs b = a;
+      const int64_t want = 4 * (int64_t)sm_count * kMinCtasBundle * kWarps;
+      b.parts = (int)std::max<int64_t>(1, std::min<int64_t>((want + bundles - 1) / bundles, (ktab_stride + kSeg - 1) / kSeg));
+      e = a.stats ? launch_persistent(march_search_bundle<true>, b, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint, bundles * b.parts)
+                  : launch_persistent(march_search_bundle<false>, b, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint, bundles * b.parts);
+    }
     mark(kKSearch);
     if (e == cudaSuccess) e = launch_queue(march_split<true>, a, ktab, ktab_stride, sm_count, s, kind);
     mark(kKSplit);

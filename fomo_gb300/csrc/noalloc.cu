@@ -168,7 +168,7 @@ extern "C" int fomo_render_noalloc(fomo_ctx* ctx, const fomo_request* req, float
   const SnapDev sd = snap_dev(snap);
   if (e == cudaSuccess) e = launch_view_init(dv, 1, s);
   if (e == cudaSuccess) e = launch_view_extents(sd, dv, 1, nullptr, s);
-  if (e == cudaSuccess) e = launch_view_finalize(dv, 1, ktab, q.nz, s);
+  if (e == cudaSuccess) e = launch_view_finalize(dv, 1, ktab, nullptr, q.nz, s);
   MarchArgs a;
   std::memset(&a, 0, sizeof(a));
   a.snap = sd;

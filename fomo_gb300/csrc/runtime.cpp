@@ -272,7 +272,7 @@ inline float ord2f(unsigned int u) {
 }
 }  // namespace
 
-GridParams choose_grid(const float* mn, const float* mx, int64_t n, double ppc) {
+GridParams choose_grid(const float* mn, const float* mx, int64_t n, double ppc, float* spacing = nullptr) {
   double ext[3], maxext = 0;
   for (int d = 0; d < 3; ++d) {
     ext[d] = (double)mx[d] - (double)mn[d];
@@ -287,6 +287,7 @@ GridParams choose_grid(const float* mn, const float* mx, int64_t n, double ppc) 
     }
   double h = ndim ? std::pow(vol * ppc / (double)std::max<int64_t>(n, 1), 1.0 / ndim) : 1.0;
   if (!(h > 0) || !std::isfinite(h)) h = 1.0;
+  if (spacing) *spacing = ndim ? (float)(h / std::pow(ppc, 1.0 / ndim)) : 0.0f;
   int dims[3];
   for (;;) {
     double cells = 1;
@@ -376,6 +377,7 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   // slower at 1 point per cell).  FOMO_CELL_OCCUPANCY sets the occupancy and
   // skips the choice.
   double ppc = ctx->cell_occupancy;
+  bool uniform = false;
   if (!ctx->occupancy_set && n >= 1024) {
     const GridParams g2 = choose_grid(mn, mx, n, 2.0);
     const int64_t nc2 = (int64_t)g2.dx * g2.dy * g2.dz;
@@ -399,9 +401,11 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
       dev_free(ctx, bits);
       return cuda_err(ctx, e, "snapshot cell statistics");
     }
-    ppc = (double)hempty < kUniformEmpty * (double)nc2 ? 1.0 : 2.0;
+    uniform = (double)hempty < kUniformEmpty * (double)nc2;
+    ppc = uniform ? 1.0 : 2.0;
   }
-  GridParams g = choose_grid(mn, mx, n, ppc);
+  float spacing = 0.0f;
+  GridParams g = choose_grid(mn, mx, n, ppc, &spacing);
   const int64_t ncells = (int64_t)g.dx * g.dy * g.dz;
   const int64_t scan_count = ncells + 1;
   const int64_t scr = exclusive_scan_scratch_ints(scan_count);
@@ -422,6 +426,8 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   R.n = n;
   R.ncells = ncells;
   R.g = g;
+  R.spacing = spacing;
+  R.uniform = uniform;
   const int bdx = (g.dx + kBlockCells - 1) / kBlockCells, bdy = (g.dy + kBlockCells - 1) / kBlockCells,
             bdz = (g.dz + kBlockCells - 1) / kBlockCells;
   const int64_t nblk = (int64_t)bdx * bdy * bdz;
@@ -726,6 +732,33 @@ std::string workload_class(const PlanGroup& G, const SnapRec& snap) {
   return k.str();
 }
 
+// Whether a view is searched as 2 x 2 blocks of rays (march_search_bundle):
+// where its pixels are at most kBundlePitch mean point spacings apart, so that
+// the rays of a block gather about the same points; farther apart, one ray
+// per warp gathers fewer.  The pitch comes from the points' bounding box,
+// rotated: the view's own extents are on the device only, and not larger.
+// All march kernels, one ray per warp against blocks (us): 2M-point loop, nz =
+// 256, pitch 1.8 spacings 606 / 646, 1.4 673 / 718, 0.9 831 / 671, 0.7 1174 / 825,
+// 0.34 3674 / 1851.  In a clustered cloud the mean spacing overstates that of its
+// dense part, where the pixels lie and the search takes longest, and the bound is
+// half that: 4M-point flux rope 1.1 1485 / 1780, 0.85 2003 / 1957, 0.43 5593 / 3709;
+// 0.5M-point rope 0.85 860 / 1047, 0.57 1137 / 1292, 0.43 1486 / 1552, 0.21 3200 / 2077.
+// Served views of kServedWhole samples or more stay with one ray per warp:
+// tests/test_gpu_failures.py cancels one 20 ms after its start and wants it to
+// run for 50 ms when it is not cancelled (41 ms as blocks).
+constexpr double kBundlePitch = 1.0, kBundlePitchClustered = 0.5;
+constexpr double kServedWhole = 1073741824.0;
+bool bundle_view(const SnapRec& snap, const fomo_request& q, int tw, int th, bool served) {
+  if ((tw | th) & 1) return false;
+  if (served && (double)q.nx * q.ny * q.nz >= kServedWhole) return false;
+  const GridParams& g = snap.g;
+  const double X = (double)g.maxx - g.minx, Y = (double)g.maxy - g.miny, Z = (double)g.maxz - g.minz;
+  const double cl = std::fabs(std::cos(q.l)), sl = std::fabs(std::sin(q.l)), cb = std::fabs(std::cos(q.b)),
+               sb = std::fabs(std::sin(q.b));
+  const double pitch = std::max((cb * cl * X + cb * sl * Y + sb * Z) / (q.nx - 1), (sl * X + cl * Y) / (q.ny - 1));
+  return pitch <= (snap.uniform ? kBundlePitch : kBundlePitchClustered) * snap.spacing;
+}
+
 // Plan a batch.  Requests are grouped into launches by (snapshot, method,
 // imaging); inside a launch, requests with the same view (angles, resolution,
 // width) become lines of one view and share the neighbour search.  All
@@ -831,6 +864,19 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
         if (ctx->rscale == 0.0f) G.rscale = t->second.rscale;
       }
     }
+    // views of coarse pixels first, those searched as blocks of rays after them; a launch with
+    // fewer segments of blocks than warps to search them takes one ray per warp (32,768 points,
+    // nz = 64: 64 x 64 pixels 33 against 49 us, 96 x 96 54 against 41)
+    const auto mid = std::stable_partition(G.vreqs.begin(), G.vreqs.end(), [&](const std::vector<int>& v) {
+      return !bundle_view(snap, reqs[v[0]], G.tw, G.th, scr->stop != nullptr);
+    });
+    G.bundle_view = (int)(mid - G.vreqs.begin());
+    int64_t units = 0;
+    for (auto v = mid; v != G.vreqs.end(); ++v) {
+      const fomo_request& q = reqs[(*v)[0]];
+      units += (int64_t)q.nx * q.ny / 4 * ((q.nz + 63) / 64);
+    }
+    if (units < 12 * (int64_t)ctx->sm_count) G.bundle_view = G.nv;
     G.o_views = L.take(sizeof(ViewDesc) * G.nv);
     G.o_lines = L.take(sizeof(LineDesc) * (size_t)G.nv * G.nl);
     G.o_off = L.take(sizeof(int64_t) * (G.nv + 1));
@@ -862,10 +908,11 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     G.o_npos = 0;
     G.o_far = 0;
     if (G.method != FOMO_METHOD_PROJECTION) {
-      const int64_t cap_items = std::max<int64_t>(1, ctx->npos_cap / G.maxnz);
+      const int64_t cap_items = std::max<int64_t>(4, ctx->npos_cap / G.maxnz & ~int64_t(3));  // whole blocks of rays
       G.npos_items = std::min<int64_t>(items, cap_items);
       G.o_npos = L.take(sizeof(int32_t) * (size_t)G.npos_items * G.maxnz);
       G.o_far = L.take(sizeof(int32_t) * (size_t)G.deferred_cap);
+      G.o_ktf = L.take(sizeof(float2) * 3 * (size_t)G.nv * G.maxnz);
     }
     G.o_s2 = G.method == FOMO_METHOD_THOMSON ? L.take(sizeof(float) * (size_t)G.nv * snap.n) : 0;
   }
@@ -1018,7 +1065,8 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
     float* s2 = G.method == FOMO_METHOD_THOMSON ? reinterpret_cast<float*>(db + G.o_s2) : nullptr;
     if (e == cudaSuccess) e = launch_view_extents(sd, dv, G.nv, s2, s);
     double3* ktab = reinterpret_cast<double3*>(db + G.o_ktab);
-    if (e == cudaSuccess) e = launch_view_finalize(dv, G.nv, ktab, G.maxnz, s);
+    float2* ktf = G.o_ktf ? reinterpret_cast<float2*>(db + G.o_ktf) : nullptr;
+    if (e == cudaSuccess) e = launch_view_finalize(dv, G.nv, ktab, ktf, G.maxnz, s);
     MarchArgs a;
     std::memset(&a, 0, sizeof(a));
     a.snap = sd;
@@ -1029,6 +1077,8 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
     a.nlines = G.nl;
     a.item_base = 0;
     a.total_items = G.total_items;
+    a.ktf = ktf;
+    a.bundle_from = G.item_off[G.bundle_view];
     a.counter = reinterpret_cast<unsigned long long*>(db + G.o_ctr);
     a.deferred = reinterpret_cast<DeferredRec*>(db + G.o_def);
     a.deferred_cap = G.deferred_cap;
@@ -1063,7 +1113,8 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
         int64_t step = G.npos_items > 0 ? G.npos_items : (i1 - i0);
         // ranges of bounded work also split a large view's rays into launches
         // of about range_cost, so that other streams' kernels start in between
-        if (range_cost > 0.0) step = std::min<int64_t>(step, std::max<int64_t>(1024, (int64_t)(range_cost / G.maxnz)));
+        if (range_cost > 0.0)
+          step = std::min<int64_t>(step, std::max<int64_t>(1024, (int64_t)(range_cost / G.maxnz) & ~int64_t(3)));
         for (int64_t b = i0; b < i1 && e == cudaSuccess; b += step) {
           if (!first) e = cudaMemsetAsync(db + G.o_ctr, 0, sizeof(unsigned long long) * kCtrCount, s);
           first = false;

@@ -44,6 +44,8 @@ struct SnapRec {
   int64_t n = 0;
   int64_t ncells = 0;
   GridParams g{};
+  float spacing = 0.0f;   // mean point spacing: (volume / points)^(1/3) over the axes with an extent
+  bool uniform = false;   // few empty cells: close to uniform at the cell scale
   void* block = nullptr;  // one allocation for everything below
   size_t bytes = 0;
   float4* pts = nullptr;
@@ -117,6 +119,8 @@ struct PlanGroup {
   size_t o_far = 0;          // slots of the records flagged for the far pass (with a neighbour buffer), or 0
   std::vector<std::pair<float*, size_t>> zero_outs;  // projection outputs to clear before the scatter
   int64_t deferred_cap = 0;  // records: one per segment of every work item
+  size_t o_ktf = 0;          // the LOS tables as FP32 pairs (with a neighbour buffer), or 0
+  int bundle_view = 0;       // views from here on are searched as 2 x 2 blocks of rays
   size_t o_hard = 0;
   int64_t hard_cap = 0;      // hard-sample queue entries
   size_t o_npos = 0;         // a neighbour per (work item, sample) for the emission pass, or 0 (projection)

@@ -312,8 +312,13 @@ __global__ void view_extents_blocks_kernel(SnapDev snap, ViewDesc* views) {
 
 __device__ __forceinline__ double dmax_ref(double a, double b) { return (a < b) ? b : a; }  // std::max
 
+__device__ __forceinline__ float2 fp32_pair(double v) {
+  const float hi = __double2float_rn(v);
+  return make_float2(hi, __double2float_rn(__dsub_rn(v, (double)hi)));
+}
+
 // One block per view.
-__global__ void view_finalize_kernel(ViewDesc* views, double3* ktab, int ktab_stride) {
+__global__ void view_finalize_kernel(ViewDesc* views, double3* ktab, float2* ktf, int ktab_stride) {
   ViewDesc* V = views + blockIdx.x;
   __shared__ double s_dz, s_minz;
   if (threadIdx.x == 0) {
@@ -375,7 +380,14 @@ __global__ void view_finalize_kernel(ViewDesc* views, double3* ktab, int ktab_st
   for (int k = threadIdx.x; k < V->nz; k += blockDim.x) {
     const double z = __dadd_rn(__dmul_rn((double)k, dz), minz);  // nn:162
     const double zsb = __dmul_rn(z, sb);
-    kt[FOMO_IDX(k, ktab_stride, kSiteKtab)] = make_double3(__dmul_rn(zsb, cl), __dmul_rn(zsb, sl), __dmul_rn(z, cb));
+    const double3 t = make_double3(__dmul_rn(zsb, cl), __dmul_rn(zsb, sl), __dmul_rn(z, cb));
+    kt[FOMO_IDX(k, ktab_stride, kSiteKtab)] = t;
+    if (ktf) {
+      float2* f = ktf + 3 * ((int64_t)blockIdx.x * ktab_stride + FOMO_IDX(k, ktab_stride, kSiteKtab));
+      f[0] = fp32_pair(t.x);
+      f[1] = fp32_pair(-t.y);
+      f[2] = fp32_pair(t.z);
+    }
   }
 }
 
@@ -411,8 +423,9 @@ cudaError_t launch_view_extents(SnapDev snap, ViewDesc* views, int nviews, float
   return cudaGetLastError();
 }
 
-cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, int ktab_stride, cudaStream_t s) {
-  view_finalize_kernel<<<nviews, 256, 0, s>>>(views, ktab, ktab_stride);
+cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, float2* ktf, int ktab_stride,
+                                 cudaStream_t s) {
+  view_finalize_kernel<<<nviews, 256, 0, s>>>(views, ktab, ktf, ktab_stride);
   return cudaGetLastError();
 }
 
