@@ -200,12 +200,13 @@ struct TableDev {
   double k;            // normaliseconst * abundratio
   int imaging;
 };
-cudaError_t launch_emission(const float* ne_s, const float* T_s, int64_t n, TableDev t, float2* ew, cudaStream_t s);
+// wmax_bits gets the largest line width of the points that emit (bits of a float >= 0).
+cudaError_t launch_emission(const float* ne_s, const float* T_s, int64_t n, TableDev t, float2* ew,
+                            unsigned int* wmax_bits, cudaStream_t s);
 cudaError_t launch_thomson_emission(const float4* pts, const float* ne_s, int64_t n, float2* totpol,
                                     cudaStream_t s);
 cudaError_t launch_unsort_payload(const float4* pts, const float2* ew, int64_t n, float* a, float* b,
                                   cudaStream_t s);
-cudaError_t launch_payload_stats(const float2* ew, int64_t n, unsigned int* wmax_bits, cudaStream_t s);
 cudaError_t launch_speed_max(const float4* vel, int64_t n, unsigned int* vmax_bits, cudaStream_t s);
 
 // view.cu

@@ -524,12 +524,11 @@ int get_payload(fomo_ctx* ctx, int snap, int table, int imaging, double abund, c
   const double normaliseconst = imaging ? 1.0 : 1. / FOMO_ALPHA;
   td.k = normaliseconst * (imaging ? 1.0 : abund);
   td.imaging = imaging;
-  cudaError_t e = launch_emission(sit->second.ne, sit->second.T, sit->second.n, td, static_cast<float2*>(p),
-                                  ctx->stream);
-  // largest line width of the emitting points: bounds the evaluated lambda window
+  // with the largest line width of the emitting points: bounds the evaluated lambda window
   unsigned int* wb = reinterpret_cast<unsigned int*>(ctx->stats_dev);
   unsigned int hw = 0x7f800000u;
-  if (e == cudaSuccess) e = launch_payload_stats(static_cast<float2*>(p), sit->second.n, wb, ctx->stream);
+  cudaError_t e = launch_emission(sit->second.ne, sit->second.T, sit->second.n, td, static_cast<float2*>(p), wb,
+                                  ctx->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&hw, wb, sizeof(hw), cudaMemcpyDeviceToHost, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
