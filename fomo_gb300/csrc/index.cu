@@ -13,6 +13,8 @@
 #include <float.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "fomo_device.cuh"
 #include "fomo_internal.h"
 
@@ -25,8 +27,13 @@ __device__ __forceinline__ unsigned int f2ord(float f) {
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
+// Six atomics per block: six per warp, 233,472 on six addresses, took 149 us of 1.4M points' whole
+// index build of 260.
 __global__ void aabb_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
                             int64_t n, unsigned int* bits6) {
+  __shared__ unsigned int sh[6];
+  if (threadIdx.x < 6) sh[threadIdx.x] = threadIdx.x < 3 ? 0xffffffffu : 0u;
+  __syncthreads();
   unsigned int mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
   unsigned int mx[3] = {0u, 0u, 0u};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -39,19 +46,19 @@ __global__ void aabb_kernel(const float* __restrict__ x, const float* __restrict
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mn[d] = min(mn[d], __shfl_xor_sync(0xffffffffu, mn[d], o));
-      mx[d] = max(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-    }
+    mn[d] = __reduce_min_sync(0xffffffffu, mn[d]);
+    mx[d] = __reduce_max_sync(0xffffffffu, mx[d]);
   }
   if ((threadIdx.x & 31) == 0) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      atomicMin(&bits6[d], mn[d]);
-      atomicMax(&bits6[3 + d], mx[d]);
+      atomicMin(&sh[d], mn[d]);
+      atomicMax(&sh[3 + d], mx[d]);
     }
   }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(&bits6[threadIdx.x], sh[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(&bits6[threadIdx.x], sh[threadIdx.x]);
 }
 
 __global__ void bin_kernel(const float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ z,
@@ -213,7 +220,7 @@ cudaError_t launch_aabb(const float* x, const float* y, const float* z, int64_t 
   if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(bits6 + 3, 0x00, 3 * sizeof(unsigned int), s);
   if (e != cudaSuccess) return e;
-  aabb_kernel<<<grid_blocks(n, 256), 256, 0, s>>>(x, y, z, n, bits6);
+  aabb_kernel<<<std::min(grid_blocks(n, 256), 152 * 4), 256, 0, s>>>(x, y, z, n, bits6);
   return cudaGetLastError();
 }
 
