@@ -25,10 +25,15 @@ std::string plan_key(const Plan& p, const ScratchSet& scr) {
   std::ostringstream k;
   k << (const void*)scr.arena.base << "/" << (const void*)scr.staging.base << "/" << p.host_bytes << "/"
     << p.dev_bytes;
-  for (const PlanGroup& G : p.groups)
+  for (const PlanGroup& G : p.groups) {
     k << "|" << G.snapshot << "," << G.method << "," << G.imaging << "," << G.nv << "," << G.nl << "," << G.maxL
       << "," << G.maxnz << "," << G.maxnx << "," << G.maxny << "," << G.total_items << "," << G.tw << "," << G.th
-      << "," << G.bps << "," << G.rscale << "," << G.any_nn << "," << G.item_off[G.bundle_view] << "," << (const void*)G.totpol;
+      << "," << G.bps << "," << G.rscale << "," << G.any_nn << "," << G.item_off[G.bundle_view] << "," << (const void*)G.totpol << "," << G.max_nw;
+    // launches that hold a view's size or an output
+    if (G.method == FOMO_METHOD_PROJECTION)
+      for (int64_t n : G.npix) k << "," << n;
+    for (const auto& z : G.zero_outs) k << "," << (const void*)z.first << ":" << z.second;
+  }
   return k.str();
 }
 

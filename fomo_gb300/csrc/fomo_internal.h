@@ -216,7 +216,22 @@ cudaError_t launch_view_extents(SnapDev snap, ViewDesc* views, int nviews, float
 cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, float2* ktf, int ktab_stride,
                                  cudaStream_t s);
 
-// projection.cu: the projection render of every view of a group (outputs zeroed beforehand)
+// projection.cu: the projection render of every view of a group with atomics (outputs zeroed beforehand),
+// or of one view by pixel (its outputs are written whole).
+bool projection_by_pixel(int64_t n, int nlines, int max_windows, bool imaging);
+int projection_pieces(int64_t n);  // capacity of ProjScratch::pieces
+struct ProjScratch {
+  int* count;               // npix + 1: points per pixel
+  int* first;               // npix + 1: their exclusive sums
+  int* scan;                // exclusive_scan_scratch_ints(npix + 1)
+  int2* at;                 // n: each point's pixel (-1: none) and its place among the pixel's
+  int* list;                // n: the points by pixel
+  int2* pieces;             // pieces of the pixels with many points
+  int pieces_cap;
+  unsigned long long* ctr;  // kCtrCount work counters
+};
+cudaError_t launch_projection_view(const ProjScratch& P, SnapDev snap, const ViewDesc* V, const LineDesc* LD, int nlines,
+                                   int max_windows, int64_t npix, int sm_count, cudaStream_t s);
 cudaError_t launch_projection(SnapDev snap, const ViewDesc* views, const LineDesc* lines, int nviews, int nlines,
                               bool imaging, int sm_count, cudaStream_t s);
 

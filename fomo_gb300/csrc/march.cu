@@ -70,6 +70,7 @@
 
 #include "fomo_device.cuh"
 #include "fomo_internal.h"
+#include "spectral_bins.cuh"
 
 namespace fomo {
 
@@ -1838,133 +1839,25 @@ __device__ __forceinline__ void walk_runs(const MarchArgs& a, const RayCtx& r, i
   __syncwarp();  // the ring is rewritten by the next ray
 }
 
-// Spectroscopy: NL lines x up to NB 32-bin windows per line.  The batch's runs
-// are staged as (peak x length, 2/w, Doppler term) per line, compacted to those
-// with a neighbour, and binned line by line and window by window: the warp is
-// four groups of eight lanes, group g adds runs g, g + 4, ... and each lane
-// evaluates four of the window's bins.  With one run for the whole warp, every
-// (run, line) cost a 16-byte broadcast to 32 lanes, 512 bytes through the shared-
-// memory port, which was the bound (22.7 ms, L1 at 85 %); a load now serves four
-// runs (18.0 ms).
-// The groups' sums are joined by an exchange that leaves bin `lane` in each
-// lane, and folded into the ray's Kahan sum.
+// Spectroscopy: SpectralBins (spectral_bins.cuh) sums the runs of one ray.
 template <int NL, int NB>
 __global__ void __launch_bounds__(kThreads, kMinCtasShade)
     march_shade_spectral(MarchArgs a, const double3* __restrict__ ktab, int ktab_stride) {
   __shared__ RunRing rings[kWarps];
-  __shared__ float4 runs[kWarps][NL][32];
-  __shared__ float lams[kWarps][NL][NB * 32];  // lambdaval (nn:200), evaluated in FP64 on the host, stored FP32
+  __shared__ BinShared<NL, NB> staged[kWarps];
   const int w = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int group = lane >> 3;
   RayCtx r;
+  SpectralBins<NL, NB> bins;
   int view = -1;
   while (next_ray(a, ktab, ktab_stride, a.total_items, r, kCtrShade)) {
     const ViewDesc* V = a.views + r.v;
-    const int L = V->L, nx = V->nx;
-    const float ux = V->ux, uy = V->uy, uz = V->uz;
     const LineDesc* LD = a.lines + (int64_t)r.v * a.nlines;
-    float acc[NL][NB], comp[NL][NB], shk[NL];
-    const float2* ew[NL];
-    int nw[NL];  // windows of the line; 0: the view has fewer lines than the launch
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      const bool on = l < a.nlines && LD[l].ew != nullptr;
-      ew[l] = on ? LD[l].ew : nullptr;
-      shk[l] = on ? LD[l].shift_k : 0.0f;
-      nw[l] = on ? min(LD[l].nw, NB) : 0;
-#pragma unroll
-      for (int m = 0; m < NB; ++m) {
-        acc[l][m] = 0.0f;
-        comp[l][m] = 0.0f;
-        if (r.v != view && m < nw[l]) {
-          const int il = LD[l].wstart + m * 32 + lane;
-          lams[w][l][m * 32 + lane] = il < L ? __ldg(LD[l].lam + FOMO_IDX(il, L, kSiteLam)) : 3.0e30f;
-        }
-      }
-    }
+    if (r.v != view) bins.view(V, LD, a.nlines, staged[w]);
     view = r.v;
-    walk_runs(a, r, ktab_stride, rings[w], [&](int m, int pos, int len) {
-      const unsigned fills = __ballot_sync(kFull, lane < m && pos >= 0);
-      const int nruns = __popc(fills);
-      if (!nruns) return;
-      const int npad = (nruns + 3) & ~3;
-      if (lane < m && pos >= 0) {
-        const float cnt = (float)len;
-        const float4 vv = __ldg(a.snap.vel + FOMO_IDX(pos, a.snap.n, kSitePts));
-        float2 pw[NL];
-#pragma unroll
-        for (int l = 0; l < NL; ++l)
-          pw[l] = nw[l] ? __ldg(ew[l] + FOMO_IDX(pos, a.snap.n, kSitePts)) : make_float2(0.0f, 1.0f);
-        const float vlos = fmaf(uz, vv.z, fmaf(uy, vv.y, ux * vv.x));
-        const int d = __popc(fills & ((1u << lane) - 1u));
-#pragma unroll
-        for (int l = 0; l < NL; ++l) {
-          // a peak of 0 (intpolpeak ? ... : 0, nn:204) is staged as all zeros and adds nothing
-          const float sc = __fdividef(2.0f, pw[l].y);  // exp(-4 ln2 (d/w)^2) = 2^(-(2d/w)^2)
-          runs[w][l][d] = pw[l].x != 0.0f ? make_float4(pw[l].x * cnt, sc, -(vlos * shk[l]) * sc, 0.0f)
-                                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
-      }
-      if (lane >= nruns && lane < npad) {
-#pragma unroll
-        for (int l = 0; l < NL; ++l) runs[w][l][lane] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      }
-      __syncwarp();
-      if (a.stats && lane == 0) {
-        int nwin = 0;
-#pragma unroll
-        for (int l = 0; l < NL; ++l) nwin += nw[l];
-        atomicAdd(a.stats + kStatRuns, (unsigned long long)nruns);
-        atomicAdd(a.stats + kStatEx2, 32ull * (unsigned long long)(nruns * nwin));
-      }
-#pragma unroll
-      for (int l = 0; l < NL; ++l) {
-#pragma unroll
-        for (int m2 = 0; m2 < NB; ++m2) {
-          if (m2 >= nw[l]) break;
-          float lam[4], part[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            lam[j] = lams[w][l][m2 * 32 + 8 * j + (lane & 7)];
-            part[j] = 0.0f;
-          }
-#pragma unroll 2
-          for (int q0 = group; q0 < npad; q0 += 4) {
-            const float4 t = runs[w][l][q0];  // the same address in the group's lanes
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float q = fmaf(lam[j], t.y, t.z);
-              part[j] = fmaf(t.x, ex2_approx(-q * q), part[j]);
-            }
-          }
-          // lane 8 g + i ends with the four groups' sum of bin 8 g + i
-          const bool hi = lane & 16, mid = lane & 8;
-          const float k0 = (hi ? part[2] : part[0]) + __shfl_xor_sync(kFull, hi ? part[0] : part[2], 16);
-          const float k1 = (hi ? part[3] : part[1]) + __shfl_xor_sync(kFull, hi ? part[1] : part[3], 16);
-          kahan_add(acc[l][m2], comp[l][m2], (mid ? k1 : k0) + __shfl_xor_sync(kFull, mid ? k0 : k1, 8));
-        }
-      }
-      __syncwarp();  // the staged runs are rewritten by the next batch
-    });
-    const int64_t ray = (int64_t)r.i * nx + r.j;
-#pragma unroll
-    for (int l = 0; l < NL; ++l) {
-      if (nw[l]) {
-        const double scale = LD[l].is_dn ? V->scale_dn : V->scale;
-        float* out = LD[l].out;
-        const int64_t ncube = (int64_t)nx * V->ny * L;
-        const int wlo = LD[l].wstart, whi = wlo + 32 * nw[l];
-        for (int il = lane; il < L; il += 32)
-          if (il < wlo || il >= whi) out[FOMO_IDX(ray * L + il, ncube, kSiteCube)] = 0.0f;  // below 2^-64 of every peak
-#pragma unroll
-        for (int m = 0; m < NB; ++m) {
-          const int il = wlo + m * 32 + lane;
-          if (m < nw[l] && il < L)
-            out[FOMO_IDX(ray * L + il, ncube, kSiteCube)] = __double2float_rn(__dmul_rn(scale, (double)acc[l][m]));
-        }
-      }
-    }
+    bins.clear();
+    walk_runs(a, r, ktab_stride, rings[w],
+              [&](int m, int pos, int len) { bins.add(a.snap, V, staged[w], m, pos, len, a.stats); });
+    bins.write(V, LD, (int64_t)r.i * V->nx + r.j);
   }
 }
 

@@ -836,6 +836,7 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
       G.maxnz = std::max(G.maxnz, q.nz);
       G.maxnx = std::max(G.maxnx, q.nx);
       G.maxny = std::max(G.maxny, q.ny);
+      G.maxnpix = std::max(G.maxnpix, (int64_t)q.nx * q.ny);
     }
     if (G.method == FOMO_METHOD_THOMSON) {
       int rc = get_thomson_payload(ctx, snap, &G.totpol);
@@ -913,6 +914,19 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
       G.o_far = L.take(sizeof(int32_t) * (size_t)G.deferred_cap);
       G.o_ktf = L.take(sizeof(float2) * 3 * (size_t)G.nv * G.maxnz);
     }
+    if (G.method == FOMO_METHOD_PROJECTION) {
+      // (the windows are known after the descriptors are filled: room for the widest lines)
+      G.by_pixel = projection_by_pixel(snap.n, G.nl, G.imaging ? 1 : (G.maxL + 31) / 32, G.imaging != 0);
+      if (G.by_pixel) {
+        const size_t npix = (size_t)G.maxnpix + 1;
+        G.o_pcount = L.take(sizeof(int) * npix);
+        G.o_pfirst = L.take(sizeof(int) * npix);
+        G.o_pscan = L.take(sizeof(int) * (size_t)exclusive_scan_scratch_ints((int64_t)npix));
+        G.o_pat = L.take(sizeof(int2) * (size_t)snap.n);
+        G.o_plist = L.take(sizeof(int) * (size_t)snap.n);
+        G.o_ppieces = L.take(sizeof(int2) * (size_t)projection_pieces(snap.n));
+      }
+    }
     G.o_s2 = G.method == FOMO_METHOD_THOMSON ? L.take(sizeof(float) * (size_t)G.nv * snap.n) : 0;
   }
   plan->dev_bytes = L.off;
@@ -971,8 +985,8 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
         }
         plan->view_of_req[r] = vbase + v;
         if (q.method == FOMO_METHOD_PROJECTION) {
-          // the projection accumulates into the output with atomics: zeroed first
-          G.zero_outs.push_back({d_out[r], sizeof(float) * cube_elems(q)});
+          // the direct projection accumulates into the output with atomics: zeroed first
+          if (!G.by_pixel) G.zero_outs.push_back({d_out[r], sizeof(float) * cube_elems(q)});
           if (d_nn && d_nn[r])
             return set_err(ctx, FOMO_EINVAL, "a projection render has no per-sample neighbour indices");
         }
@@ -984,6 +998,9 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     }
     G.total_items = hoff[G.nv];
     G.item_off.assign(hoff, hoff + G.nv + 1);
+    G.npix.clear();
+    for (int v = 0; v < G.nv; ++v)
+      G.npix.push_back((int64_t)reqs[G.vreqs[v][0]].nx * reqs[G.vreqs[v][0]].ny);
     G.vcost.assign(G.nv, 0.0);
     G.out_bytes = 0;
     for (int v = 0; v < G.nv; ++v) {
@@ -1098,7 +1115,21 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
     if (G.method == FOMO_METHOD_PROJECTION) {
       for (const auto& z : G.zero_outs)
         if (e == cudaSuccess) e = cudaMemsetAsync(z.first, 0, z.second, s);
-      if (e == cudaSuccess) e = launch_projection(sd, dv, a.lines, G.nv, G.nl, G.imaging, ctx->sm_count, s);
+      if (G.by_pixel) {
+        ProjScratch P;
+        P.count = reinterpret_cast<int*>(db + G.o_pcount);
+        P.first = reinterpret_cast<int*>(db + G.o_pfirst);
+        P.scan = reinterpret_cast<int*>(db + G.o_pscan);
+        P.at = reinterpret_cast<int2*>(db + G.o_pat);
+        P.list = reinterpret_cast<int*>(db + G.o_plist);
+        P.pieces = reinterpret_cast<int2*>(db + G.o_ppieces);
+        P.pieces_cap = projection_pieces(snap.n);
+        P.ctr = a.counter;
+        for (int v = 0; v < G.nv && e == cudaSuccess; ++v)
+          e = launch_projection_view(P, sd, dv + v, a.lines + (size_t)v * G.nl, G.nl, G.max_nw, G.npix[v], ctx->sm_count, s);
+      } else if (e == cudaSuccess) {
+        e = launch_projection(sd, dv, a.lines, G.nv, G.nl, G.imaging, ctx->sm_count, s);
+      }
       if (e == cudaSuccess && done) rc = (*done)(G, 0, G.nv);
     } else if (e == cudaSuccess) {
       // the march over view ranges: each range's rays are a contiguous run of

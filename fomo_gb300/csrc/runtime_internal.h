@@ -118,6 +118,8 @@ struct PlanGroup {
   size_t o_def = 0;          // deferred-sample records
   size_t o_far = 0;          // slots of the records flagged for the far pass (with a neighbour buffer), or 0
   std::vector<std::pair<float*, size_t>> zero_outs;  // projection outputs to clear before the scatter
+  bool by_pixel = false;     // a projection that lists its points by pixel, view by view
+  size_t o_pcount = 0, o_pfirst = 0, o_pscan = 0, o_pat = 0, o_plist = 0, o_ppieces = 0;
   int64_t deferred_cap = 0;  // records: one per segment of every work item
   size_t o_ktf = 0;          // the LOS tables as FP32 pairs (with a neighbour buffer), or 0
   int bundle_view = 0;       // views from here on are searched as 2 x 2 blocks of rays
@@ -125,6 +127,8 @@ struct PlanGroup {
   int64_t hard_cap = 0;      // hard-sample queue entries
   size_t o_npos = 0;         // a neighbour per (work item, sample) for the emission pass, or 0 (projection)
   int64_t npos_items = 0;    // work items the neighbour buffer holds (the launch marches in chunks of these)
+  int64_t maxnpix = 4;            // pixels of the largest view
+  std::vector<int64_t> npix;      // pixels of each view
   std::vector<int64_t> item_off;  // first work item of each view (nv + 1 entries)
   std::vector<double> vcost;      // LOS samples + output cells of each view
   size_t out_bytes = 0;           // cube bytes of all its requests
