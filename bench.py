@@ -581,10 +581,10 @@ def run_ours(args):
             "clocks": clocks,
             "ceilings": ceilings,
             "kernels": kernels,
-            # per step: view init, view bounds (per block of cells), view extents (the blocks that can hold an
-            # extreme), view finalize, search, overflow split, far pass, deferred march, hard-sample march,
+            # per step: view bounds (per block of cells), view extents (the blocks that can hold an
+            # extreme), view finalize, search, overflow split, deferred march,
             # emission
-            "gpu_launches": 10 * args.steps,
+            "gpu_launches": 7 * args.steps,
             "serving": serving,
         }
         print(json.dumps(out))

@@ -48,7 +48,7 @@ struct ViewDesc {
   int method;
   int is_dn;
   int ray_tile_w, ray_tile_h;  // ray tile shape for the march work order
-  // ---- device-filled by the extents + finalize kernels
+  // ---- device-filled by the extents + finalize kernels (ext_bits and bnd start from the host's fill)
   unsigned long long ext_bits[6];  // order-preserving encodings for atomic min/max
   int bnd[6];                // per rotated axis: the largest lower bound of a block's values and the smallest
                              // upper bound (order-preserving float encodings), which bound the extremes
@@ -93,6 +93,9 @@ enum MarchCounter {
   kCtrFar, kCtrFarHead, kCtrBundles,
   kCtrCount
 };
+
+// Box half-width, in cells, from which the far pass takes a view's samples (narrower: lane walks).
+constexpr float kFarBox = 4.0f;
 
 // One segment whose samples the march's first search pass could not resolve:
 // x = work item of the ray, y = first LOS sample of the segment (bits 0-29;
@@ -210,11 +213,11 @@ cudaError_t launch_unsort_payload(const float4* pts, const float2* ew, int64_t n
 cudaError_t launch_speed_max(const float4* vel, int64_t n, unsigned int* vmax_bits, cudaStream_t s);
 
 // view.cu
-cudaError_t launch_view_init(ViewDesc* views, int nviews, cudaStream_t s);
 cudaError_t launch_view_extents(SnapDev snap, ViewDesc* views, int nviews, float* s2, cudaStream_t s);
-// ktf (null: not wanted) gets the LOS table as FP32 pairs, three per sample.
+// ktf (null: not wanted) gets the LOS table as FP32 pairs, three per sample; max_entries: the largest
+// nx + ny + nz of the views.
 cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, float2* ktf, int ktab_stride,
-                                 cudaStream_t s);
+                                 int max_entries, cudaStream_t s);
 
 // projection.cu: the projection render of every view of a group with atomics (outputs zeroed beforehand),
 // or of one view by pixel (its outputs are written whole).

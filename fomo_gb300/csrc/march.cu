@@ -97,7 +97,6 @@ constexpr float kRScaleDefault = 0.9f;  // gather radius in local point spacings
 // kFarMin or more of them in a half record, searched together by a warp.
 constexpr int kFarMin = 4;          // far samples a half needs (fewer: the lane walks of march_deferred)
 constexpr float kFarOut2 = 0.25f;   // squared distance, in cells, off the points' bounding box of a far sample
-constexpr float kFarBox = 4.0f;     // box half-width, in cells, of the views the far pass takes (narrower: lane walks)
 constexpr int kFarIters = 4;        // gathers per half
 constexpr int kFarMaxPts = 1024;    // points of a gather beyond which the half is left to march_deferred
 // A deferred record is (work item, first sample of its 64-sample segment with
@@ -3044,7 +3043,7 @@ cudaError_t launch_march(const MarchArgs& a, const double3* ktab, int ktab_strid
     mark(kKSearch);
     if (e == cudaSuccess) e = launch_queue(march_split<true>, a, ktab, ktab_stride, sm_count, s, kind);
     mark(kKSplit);
-    if (e == cudaSuccess) e = launch_queue(march_far, a, ktab, ktab_stride, sm_count, s, kind);
+    if (e == cudaSuccess && a.far_list) e = launch_queue(march_far, a, ktab, ktab_stride, sm_count, s, kind);
     mark(kKFar);
     if (e == cudaSuccess) e = launch_queue(march_deferred<true>, a, ktab, ktab_stride, sm_count, s, kind);
     mark(kKDeferred);

@@ -166,9 +166,8 @@ extern "C" int fomo_render_noalloc(fomo_ctx* ctx, const fomo_request* req, float
   put_header<<<1, 128, 0, s>>>(blob, reinterpret_cast<uint4*>(base));
   e = cudaGetLastError();
   const SnapDev sd = snap_dev(snap);
-  if (e == cudaSuccess) e = launch_view_init(dv, 1, s);
   if (e == cudaSuccess) e = launch_view_extents(sd, dv, 1, nullptr, s);
-  if (e == cudaSuccess) e = launch_view_finalize(dv, 1, ktab, nullptr, q.nz, s);
+  if (e == cudaSuccess) e = launch_view_finalize(dv, 1, ktab, nullptr, q.nz, q.nx + q.ny + q.nz, s);
   MarchArgs a;
   std::memset(&a, 0, sizeof(a));
   a.snap = sd;

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cctype>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -674,6 +675,12 @@ void fill_view_host(const fomo_request& q, double lambda0, int tw, int th, ViewD
               : (q.method == FOMO_METHOD_PROJECTION ? kMethodProjection : kMethodNN);
   V->ray_tile_w = tw;
   V->ray_tile_h = th;
+  for (int d = 0; d < 3; ++d) {
+    V->ext_bits[2 * d] = ~0ull;         // min
+    V->ext_bits[2 * d + 1] = 0ull;      // max
+    V->bnd[2 * d] = INT_MIN;            // largest lower bound (atomicMax)
+    V->bnd[2 * d + 1] = INT_MAX;        // smallest upper bound (atomicMin)
+  }
 }
 
 void view_info_from(const ViewDesc& V, const fomo_request& q, const TableHost* t, fomo_view_info* info) {
@@ -731,12 +738,20 @@ std::string workload_class(const PlanGroup& G, const SnapRec& snap) {
   return k.str();
 }
 
+// The larger pixel pitch of a view from the points' bounding box, rotated: at
+// least the view's own (its extents are on the device only, and not larger).
+double view_pitch(const SnapRec& snap, const fomo_request& q) {
+  const GridParams& g = snap.g;
+  const double X = (double)g.maxx - g.minx, Y = (double)g.maxy - g.miny, Z = (double)g.maxz - g.minz;
+  const double cl = std::fabs(std::cos(q.l)), sl = std::fabs(std::sin(q.l)), cb = std::fabs(std::cos(q.b)),
+               sb = std::fabs(std::sin(q.b));
+  return std::max((cb * cl * X + cb * sl * Y + sb * Z) / (q.nx - 1), (sl * X + cl * Y) / (q.ny - 1));
+}
+
 // Whether a view is searched as 2 x 2 blocks of rays (march_search_bundle):
 // where its pixels are at most kBundlePitch mean point spacings apart, so that
 // the rays of a block gather about the same points; farther apart, one ray
-// per warp gathers fewer.  The pitch comes from the points' bounding box,
-// rotated: the view's own extents are on the device only, and not larger.
-// All march kernels, one ray per warp against blocks (us): 2M-point loop, nz =
+// per warp gathers fewer.  All march kernels, one ray per warp against blocks (us): 2M-point loop, nz =
 // 256, pitch 1.8 spacings 606 / 646, 1.4 673 / 718, 0.9 831 / 671, 0.7 1174 / 825,
 // 0.34 3674 / 1851.  In a clustered cloud the mean spacing overstates that of its
 // dense part, where the pixels lie and the search takes longest, and the bound is
@@ -750,12 +765,7 @@ constexpr double kServedWhole = 1073741824.0;
 bool bundle_view(const SnapRec& snap, const fomo_request& q, int tw, int th, bool served) {
   if ((tw | th) & 1) return false;
   if (served && (double)q.nx * q.ny * q.nz >= kServedWhole) return false;
-  const GridParams& g = snap.g;
-  const double X = (double)g.maxx - g.minx, Y = (double)g.maxy - g.miny, Z = (double)g.maxz - g.minz;
-  const double cl = std::fabs(std::cos(q.l)), sl = std::fabs(std::sin(q.l)), cb = std::fabs(std::cos(q.b)),
-               sb = std::fabs(std::sin(q.b));
-  const double pitch = std::max((cb * cl * X + cb * sl * Y + sb * Z) / (q.nx - 1), (sl * X + cl * Y) / (q.ny - 1));
-  return pitch <= (snap.uniform ? kBundlePitch : kBundlePitchClustered) * snap.spacing;
+  return view_pitch(snap, q) <= (snap.uniform ? kBundlePitch : kBundlePitchClustered) * snap.spacing;
 }
 
 // Plan a batch.  Requests are grouped into launches by (snapshot, method,
@@ -884,13 +894,13 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     size_t lam_total = 0;
     for (auto& v : G.vreqs) lam_total += (size_t)v.size() * (size_t)G.maxL;
     G.o_lam = L.take(sizeof(float) * std::max<size_t>(lam_total, 1));
+    G.o_ctr = L.take(sizeof(unsigned long long) * kCtrCount);  // the upload clears them
   }
   plan->host_bytes = L.off;  // the staged (uploaded) part
   for (PlanGroup& G : plan->groups) {
     SnapRec& snap = ctx->snaps[G.snapshot];
     G.o_ktab = L.take(sizeof(double3) * (size_t)G.nv * G.maxnz);
     G.o_xy = L.take(sizeof(double) * (size_t)G.nv * (G.maxnx + G.maxny));
-    G.o_ctr = L.take(sizeof(unsigned long long) * kCtrCount);
     int64_t items = 0;
     for (auto& v : G.vreqs) {
       const fomo_request& q = reqs[v[0]];
@@ -898,7 +908,13 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     }
     G.deferred_cap = deferred_capacity(items, G.maxnz);
     G.o_def = L.take(sizeof(DeferredRec) * (size_t)G.deferred_cap);
-    G.hard_cap = hard_capacity(items, G.maxnz);
+    // Boxes narrower than kFarBox cells in every view (md = pitch / 0.3, nn:138): no half record
+    // can be listed for the far pass.  In a cloud close to uniform a lane's walk over such a box
+    // is short as well, and needs no queue of hard samples.  Either pass is a launch of 3 to 5 us
+    // that finds its queue empty.
+    bool wide = G.method == FOMO_METHOD_THOMSON;
+    for (auto& v : G.vreqs) wide = wide || view_pitch(snap, reqs[v[0]]) / 0.3 * 1.0001 >= kFarBox * snap.g.h;
+    G.hard_cap = wide || !snap.uniform ? hard_capacity(items, G.maxnz) : 0;
     G.o_hard = L.take(sizeof(uint2) * (size_t)G.hard_cap);
     // the searches and the emission run as separate passes through a
     // neighbour buffer (each pass at its own occupancy; the emission pass runs
@@ -911,7 +927,7 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
       const int64_t cap_items = std::max<int64_t>(4, ctx->npos_cap / G.maxnz & ~int64_t(3));  // whole blocks of rays
       G.npos_items = std::min<int64_t>(items, cap_items);
       G.o_npos = L.take(sizeof(int32_t) * (size_t)G.npos_items * G.maxnz);
-      G.o_far = L.take(sizeof(int32_t) * (size_t)G.deferred_cap);
+      if (wide) G.o_far = L.take(sizeof(int32_t) * (size_t)G.deferred_cap);
       G.o_ktf = L.take(sizeof(float2) * 3 * (size_t)G.nv * G.maxnz);
     }
     if (G.method == FOMO_METHOD_PROJECTION) {
@@ -1074,15 +1090,13 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
   for (const PlanGroup& G : plan.groups) {
     if (e != cudaSuccess) break;
     SnapRec& snap = ctx->snaps[G.snapshot];
-    e = cudaMemsetAsync(db + G.o_ctr, 0, sizeof(unsigned long long) * kCtrCount, s);
     ViewDesc* dv = reinterpret_cast<ViewDesc*>(db + G.o_views);
-    if (e == cudaSuccess) e = launch_view_init(dv, G.nv, s);
     SnapDev sd = snap_dev(snap);
     float* s2 = G.method == FOMO_METHOD_THOMSON ? reinterpret_cast<float*>(db + G.o_s2) : nullptr;
     if (e == cudaSuccess) e = launch_view_extents(sd, dv, G.nv, s2, s);
     double3* ktab = reinterpret_cast<double3*>(db + G.o_ktab);
     float2* ktf = G.o_ktf ? reinterpret_cast<float2*>(db + G.o_ktf) : nullptr;
-    if (e == cudaSuccess) e = launch_view_finalize(dv, G.nv, ktab, ktf, G.maxnz, s);
+    if (e == cudaSuccess) e = launch_view_finalize(dv, G.nv, ktab, ktf, G.maxnz, G.maxnx + G.maxny + G.maxnz, s);
     MarchArgs a;
     std::memset(&a, 0, sizeof(a));
     a.snap = sd;
