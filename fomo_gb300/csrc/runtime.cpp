@@ -126,7 +126,7 @@ void release_free_blocks(fomo_ctx* ctx) {
   ctx->cached = 0;
 }
 
-void dev_free(fomo_ctx* ctx, void* p) {
+void dev_free(fomo_ctx* ctx, void* p, bool idle) {
   if (!p) return;
   auto it = ctx->sizes.find(p);
   size_t bytes = 0;
@@ -138,7 +138,7 @@ void dev_free(fomo_ctx* ctx, void* p) {
   if (bytes > 0 && bytes <= kKeepBlock && ctx->cached + bytes <= kKeepTotal) {
     // kept for the next allocation of the same size instead of unmapped and
     // mapped again; like cudaFree, only once the device is done with it
-    cudaDeviceSynchronize();
+    if (!idle) cudaDeviceSynchronize();
     ctx->free_blocks.emplace(bytes, p);
     ctx->cached += bytes;
     return;
@@ -168,6 +168,25 @@ int Arena::reserve(fomo_ctx* ctx, size_t bytes) {
   base = static_cast<char*>(p);
   cap = want;
   return FOMO_OK;
+}
+
+// Pinned memory for `bytes` (at most kBounceMax), or null: the caller then copies without it.
+constexpr size_t kBounceMax = size_t(1) << 20;
+char* bounce_buffer(fomo_ctx* ctx, size_t bytes) {
+  if (bytes > kBounceMax) return nullptr;
+  if (bytes > ctx->bounce_cap) {
+    if (ctx->bounce) cudaFreeHost(ctx->bounce);
+    ctx->bounce = nullptr;
+    ctx->bounce_cap = 0;
+    const size_t want = std::max<size_t>(bytes, 64 << 10);
+    if (cudaMallocHost(reinterpret_cast<void**>(&ctx->bounce), want) != cudaSuccess) {
+      cudaGetLastError();
+      ctx->bounce = nullptr;
+      return nullptr;
+    }
+    ctx->bounce_cap = want;
+  }
+  return ctx->bounce;
 }
 
 int Staging::reserve(fomo_ctx* ctx, size_t bytes) {
@@ -320,28 +339,52 @@ GridParams choose_grid(const float* mn, const float* mx, int64_t n, double ppc, 
   return g;
 }
 
+// `bytes` at device address src to dst, waited for.  Through pinned memory: a copy to pageable
+// memory takes a few us more.
+cudaError_t read_back(fomo_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  char* p = bounce_buffer(ctx, bytes);
+  cudaError_t e = cudaMemcpyAsync(p ? p : dst, src, bytes, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && p) std::memcpy(dst, p, bytes);
+  return e;
+}
+
 constexpr double kUniformEmpty = 0.10;  // empty-cell share below which a cloud counts as uniform
 
 int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec* out) {
   NvtxRange range("fomo: snapshot upload and index");
   cudaStream_t s = ctx->stream;
-  // staging: 8 arrays of n floats (z may be absent -> zeros, as nn:82 for 2-D data)
-  float* stage = nullptr;
-  int rc = dev_alloc(ctx, reinterpret_cast<void**>(&stage), sizeof(float) * 8 * (size_t)n);
-  if (rc) return rc;
-  float* a[8];
-  for (int k = 0; k < 8; ++k) a[k] = stage + (size_t)k * n;
+  // staging for the host arrays (z may be absent -> zeros, as nn:82 for 2-D data); arrays in this
+  // device's memory are read where they are
+  const float* a[8];
+  int nstage = 0;
   for (int k = 0; k < 8; ++k) {
+    a[k] = nullptr;
+    cudaPointerAttributes at;
+    if (host[k] && cudaPointerGetAttributes(&at, host[k]) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+        at.device == ctx->device)
+      a[k] = host[k];
+    else
+      ++nstage;
+  }
+  cudaGetLastError();  // a plain host pointer may be an error to the query
+  float* stage = nullptr;
+  int rc = dev_alloc(ctx, reinterpret_cast<void**>(&stage), sizeof(float) * (size_t)nstage * (size_t)n);
+  if (rc) return rc;
+  float* put = stage;
+  for (int k = 0; k < 8; ++k) {
+    if (a[k]) continue;
+    a[k] = put;
     if (host[k]) {
-      // host or device memory alike (unified addressing: a device array is copied on the device)
-      cudaError_t e = cudaMemcpyAsync(a[k], host[k], sizeof(float) * n, cudaMemcpyDefault, s);
+      cudaError_t e = cudaMemcpyAsync(put, host[k], sizeof(float) * n, cudaMemcpyDefault, s);
       if (e != cudaSuccess) {
         dev_free(ctx, stage);
         return cuda_err(ctx, e, "snapshot upload");
       }
     } else {
-      cudaMemsetAsync(a[k], 0, sizeof(float) * n, s);
+      cudaMemsetAsync(put, 0, sizeof(float) * n, s);
     }
+    put += n;
   }
   unsigned int* bits = nullptr;
   rc = dev_alloc(ctx, reinterpret_cast<void**>(&bits), 64);
@@ -351,8 +394,7 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   }
   unsigned int hb[6];
   cudaError_t e = launch_aabb(a[0], a[1], a[2], n, bits, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hb, bits, sizeof(hb), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = read_back(ctx, hb, bits, sizeof(hb), s);
   if (e != cudaSuccess) {
     dev_free(ctx, stage);
     dev_free(ctx, bits);
@@ -394,9 +436,8 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
     e = cudaMemsetAsync(t2 + n, 0, sizeof(int) * (size_t)nc2, s);
     if (e == cudaSuccess) e = launch_bin_points(a[0], a[1], a[2], n, g2, t2, t2 + n, s);
     if (e == cudaSuccess) e = launch_count_empty(t2 + n, nc2, dempty, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hempty, dempty, sizeof(hempty), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    dev_free(ctx, t2);
+    if (e == cudaSuccess) e = read_back(ctx, &hempty, dempty, sizeof(hempty), s);
+    dev_free(ctx, t2, e == cudaSuccess);
     if (e != cudaSuccess) {
       dev_free(ctx, stage);
       dev_free(ctx, bits);
@@ -464,12 +505,13 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   if (e == cudaSuccess) e = launch_block_bounds(R.pts, R.cell_start, g, bdx, bdy, bdz, R.blk, s);
   unsigned int vbits = 0x7f800000u;
   if (e == cudaSuccess) e = launch_speed_max(R.vel, n, bits, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&vbits, bits, sizeof(vbits), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess) e = read_back(ctx, &vbits, bits, sizeof(vbits), s);
   std::memcpy(&R.vmax, &vbits, sizeof(R.vmax));
-  dev_free(ctx, stage);
-  dev_free(ctx, bits);
-  dev_free(ctx, tmp);
+  // (only this stream has used them, and it is done)
+  const bool idle = e == cudaSuccess;
+  dev_free(ctx, stage, idle);
+  dev_free(ctx, bits, idle);
+  dev_free(ctx, tmp, idle);
   if (e != cudaSuccess) {
     dev_free(ctx, res);
     return cuda_err(ctx, e, "snapshot index build");
@@ -492,55 +534,78 @@ SnapDev snap_dev(const SnapRec& r) {
   return s;
 }
 
-// Emissivity payload for (snapshot, table, observation type, abundance),
+// Emissivity payloads for (snapshot, table, observation type, abundance), each
 // computed once and kept resident (the reference recomputes it on every
-// render, fomo-object.cpp:389-400).
-int get_payload(fomo_ctx* ctx, int snap, int table, int imaging, double abund, const float2** out) {
-  NvtxRange range("fomo: emissivity");
-  auto key = std::make_tuple(snap, table, imaging, abund);
-  auto it = ctx->payloads.find(key);
-  if (it != ctx->payloads.end()) {
-    *out = it->second;
-    return FOMO_OK;
-  }
-  auto sit = ctx->snaps.find(snap);
-  if (sit == ctx->snaps.end()) return set_err(ctx, FOMO_ENOTFOUND, "unknown snapshot id");
-  auto tit = ctx->tables.find(table);
-  if (tit == ctx->tables.end()) return set_err(ctx, FOMO_ENOTFOUND, "unknown table id");
-  const TableHost& th = tit->second.h;
-  if (imaging && std::atoi(th.ion.c_str()) != (int)(th.lambda0 + 0.5))
-    return set_err(ctx, FOMO_ETABLE, "GOFT table is not correct! (imaging needs atoi(ion) == int(lambda0+0.5))");
-  void* p = nullptr;
-  int rc = dev_alloc(ctx, &p, sizeof(float2) * (size_t)sit->second.n);
-  if (rc) return rc;
-  TableDev td;
-  td.nt = th.nt;
-  td.nrho = th.nrho;
-  td.logT = tit->second.d;
-  td.logn = tit->second.d + th.nt;
-  td.G = tit->second.d + th.nt + th.nrho;
-  // linefwhm constant (fomo-CHIANTI.cpp:224), same expression order
-  td.cw = 2 * std::sqrt(2 * std::log(2)) * std::sqrt(FOMO_BOLTZMANN / FOMO_MASS_PROTON / th.atweight) * th.lambda0 /
-          FOMO_SPEED_OF_LIGHT;
-  const double normaliseconst = imaging ? 1.0 : 1. / FOMO_ALPHA;
-  td.k = normaliseconst * (imaging ? 1.0 : abund);
-  td.imaging = imaging;
-  // with the largest line width of the emitting points: bounds the evaluated lambda window
+// render, fomo-object.cpp:389-400).  Those that `keys` lacks are computed one
+// after the other and their largest line widths, which bound the evaluated lambda
+// windows, read back together (one synchronize, not one per table).
+using PayloadKey = std::tuple<int, int, int, double>;
+int ensure_payloads(fomo_ctx* ctx, const std::vector<PayloadKey>& keys) {
+  std::vector<std::pair<PayloadKey, void*>> made;
+  int rc = FOMO_OK;
+  cudaError_t e = cudaSuccess;
+  constexpr size_t kWords = 64;  // of stats_dev
   unsigned int* wb = reinterpret_cast<unsigned int*>(ctx->stats_dev);
-  unsigned int hw = 0x7f800000u;
-  cudaError_t e = launch_emission(sit->second.ne, sit->second.T, sit->second.n, td, static_cast<float2*>(p), wb,
-                                  ctx->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hw, wb, sizeof(hw), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  for (const PayloadKey& key : keys) {
+    if (ctx->payloads.count(key) || made.size() == kWords) continue;
+    bool have = false;
+    for (auto& m : made) have = have || m.first == key;
+    if (have) continue;
+    const int snap = std::get<0>(key), table = std::get<1>(key), imaging = std::get<2>(key);
+    auto sit = ctx->snaps.find(snap);
+    auto tit = ctx->tables.find(table);
+    if (sit == ctx->snaps.end()) rc = set_err(ctx, FOMO_ENOTFOUND, "unknown snapshot id");
+    else if (tit == ctx->tables.end()) rc = set_err(ctx, FOMO_ENOTFOUND, "unknown table id");
+    else if (imaging && std::atoi(tit->second.h.ion.c_str()) != (int)(tit->second.h.lambda0 + 0.5))
+      rc = set_err(ctx, FOMO_ETABLE, "GOFT table is not correct! (imaging needs atoi(ion) == int(lambda0+0.5))");
+    if (rc) break;
+    const TableHost& th = tit->second.h;
+    void* p = nullptr;
+    rc = dev_alloc(ctx, &p, sizeof(float2) * (size_t)sit->second.n);
+    if (rc) break;
+    TableDev td;
+    td.nt = th.nt;
+    td.nrho = th.nrho;
+    td.logT = tit->second.d;
+    td.logn = tit->second.d + th.nt;
+    td.G = tit->second.d + th.nt + th.nrho;
+    // linefwhm constant (fomo-CHIANTI.cpp:224), same expression order
+    td.cw = 2 * std::sqrt(2 * std::log(2)) * std::sqrt(FOMO_BOLTZMANN / FOMO_MASS_PROTON / th.atweight) * th.lambda0 /
+            FOMO_SPEED_OF_LIGHT;
+    const double normaliseconst = imaging ? 1.0 : 1. / FOMO_ALPHA;
+    td.k = normaliseconst * (imaging ? 1.0 : std::get<3>(key));
+    td.imaging = imaging;
+    made.emplace_back(key, p);
+    e = launch_emission(sit->second.ne, sit->second.T, sit->second.n, td, static_cast<float2*>(p), wb + made.size() - 1,
+                        ctx->stream);
+    if (e != cudaSuccess) break;
+  }
+  if (made.empty()) return rc;
+  unsigned int hw[kWords];
+  if (e == cudaSuccess) e = read_back(ctx, hw, wb, sizeof(unsigned int) * made.size(), ctx->stream);
   if (e != cudaSuccess) {
-    dev_free(ctx, p);
+    for (auto& m : made) dev_free(ctx, m.second);
     return cuda_err(ctx, e, "emission kernel");
   }
-  float wmax;
-  std::memcpy(&wmax, &hw, sizeof(wmax));
-  ctx->payloads[key] = static_cast<float2*>(p);
-  ctx->payload_wmax[key] = imaging ? 1.0f : wmax;
-  *out = static_cast<float2*>(p);
+  for (size_t i = 0; i < made.size(); ++i) {
+    float wmax;
+    std::memcpy(&wmax, &hw[i], sizeof(wmax));
+    ctx->payloads[made[i].first] = static_cast<float2*>(made[i].second);
+    ctx->payload_wmax[made[i].first] = std::get<2>(made[i].first) ? 1.0f : wmax;
+  }
+  return rc;
+}
+
+int get_payload(fomo_ctx* ctx, int snap, int table, int imaging, double abund, const float2** out) {
+  NvtxRange range("fomo: emissivity");
+  const PayloadKey key(snap, table, imaging, abund);
+  auto it = ctx->payloads.find(key);
+  if (it == ctx->payloads.end()) {
+    int rc = ensure_payloads(ctx, {key});
+    if (rc) return rc;
+    it = ctx->payloads.find(key);
+  }
+  *out = it->second;
   return FOMO_OK;
 }
 
@@ -813,6 +878,21 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     std::stable_sort(plan->groups.begin(), plan->groups.end(),
                      [&](const PlanGroup& a, const PlanGroup& b) { return work(a) < work(b); });
   }
+  {
+    // the emissivities that the batch lacks, together
+    std::vector<PayloadKey> keys;
+    for (const PlanGroup& G : plan->groups)
+      if (G.method != FOMO_METHOD_THOMSON)
+        for (int r : G.reqs) {
+          const PayloadKey key(G.snapshot, reqs[r].table, G.imaging, reqs[r].abundratio);
+          if (!ctx->payloads.count(key)) keys.push_back(key);
+        }
+    if (!keys.empty()) {
+      NvtxRange er("fomo: emissivity");
+      const int rc = ensure_payloads(ctx, keys);
+      if (rc) return rc;
+    }
+  }
   Layout L;
   const size_t hdr = L.take(0);
   (void)hdr;
@@ -1042,7 +1122,7 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
 // view set-up and the persistent march.
 // Cut points [0 = c0 < c1 < ... = nv] of the view ranges a launch marches in
 // when its cubes download as they complete: about equal shares of the views'
-// cost, one range per 256 MB of cubes, 8 at most.
+// cost, one range per 64 MB of cubes, 8 at most.
 static std::vector<int> view_ranges(const PlanGroup& G, bool split, double range_cost) {
   if (split && range_cost > 0.0) {
     // ranges of about range_cost each (views in plan order: smaller images first)
@@ -1058,7 +1138,7 @@ static std::vector<int> view_ranges(const PlanGroup& G, bool split, double range
     cuts.push_back(G.nv);
     return cuts;
   }
-  const size_t n = split ? std::min<size_t>({8, (size_t)G.nv, std::max<size_t>(1, G.out_bytes >> 28)}) : 1;
+  const size_t n = split ? std::min<size_t>({8, (size_t)G.nv, std::max<size_t>(1, G.out_bytes >> 26)}) : 1;
   double total = 0.0;
   for (double c : G.vcost) total += c;
   std::vector<int> cuts{0};
@@ -1189,9 +1269,9 @@ int enqueue_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* cons
   rc = issue_plan(ctx, plan, &ctx->scratch, s, done);
   if (rc) return rc;
   if (view_of_req) *view_of_req = plan.view_of_req;
+  ctx->view_readback.clear();
   if (views_out) {
     views_out->assign(plan.nviews_total, ViewDesc{});
-    ctx->view_readback.clear();
     for (const PlanGroup& G : plan.groups)
       ctx->view_readback.push_back({reinterpret_cast<ViewDesc*>(ctx->scratch.arena.base + G.o_views),
                                     (size_t)G.vbase, G.nv});
@@ -1225,16 +1305,27 @@ void load_tune_cache(fomo_ctx* ctx, const char* path) {
   }
 }
 
-int finish_views(fomo_ctx* ctx, std::vector<ViewDesc>* views) {
+// The views of the last batch into `at` (pinned memory, or the caller's), on stream s; after
+// that stream is waited for, take_views copies them out.
+size_t views_bytes(const fomo_ctx* ctx) {
+  size_t b = 0;
+  for (auto& rb : ctx->view_readback) b += sizeof(ViewDesc) * rb.count;
+  return b;
+}
+cudaError_t queue_views(fomo_ctx* ctx, char* at, cudaStream_t s) {
+  cudaError_t e = cudaSuccess;
   for (auto& rb : ctx->view_readback) {
-    cudaError_t e = cudaMemcpy(views->data() + rb.base, rb.dev, sizeof(ViewDesc) * rb.count, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) {
-      ctx->view_readback.clear();
-      return cuda_err(ctx, e, "view readback");
-    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(at, rb.dev, sizeof(ViewDesc) * rb.count, cudaMemcpyDeviceToHost, s);
+    at += sizeof(ViewDesc) * rb.count;
+  }
+  return e;
+}
+void take_views(fomo_ctx* ctx, const char* at, std::vector<ViewDesc>* views) {
+  for (auto& rb : ctx->view_readback) {
+    std::memcpy(views->data() + rb.base, at, sizeof(ViewDesc) * rb.count);
+    at += sizeof(ViewDesc) * rb.count;
   }
   ctx->view_readback.clear();
-  return FOMO_OK;
 }
 
 }  // namespace fomo
@@ -1313,6 +1404,7 @@ int fomo_ctx_destroy(fomo_ctx* ctx) {
   dev_free(ctx, ctx->out_arena.base);
   release_free_blocks(ctx);
   if (ctx->stats_dev) cudaFree(ctx->stats_dev);
+  if (ctx->bounce) cudaFreeHost(ctx->bounce);
   if (ctx->timer.ev) {
     for (int i = 0; i < ctx->timer.cap; ++i) cudaEventDestroy(ctx->timer.ev[i]);
     delete[] ctx->timer.ev;
@@ -1543,11 +1635,12 @@ int fomo_render_device(fomo_ctx* ctx, const fomo_request* req, float* d_out_cube
   int rc = enqueue_batch(ctx, req, 1, outs, nns, s, info ? &views : nullptr, &vof);
   if (rc) return rc;
   if (info) {
+    std::vector<char> buf(views_bytes(ctx));
+    FOMO_CUDA(queue_views(ctx, buf.data(), s), "view readback");
     FOMO_CUDA(cudaStreamSynchronize(s), "render");
     rc = check_device_words(ctx);
     if (rc) return rc;
-    rc = finish_views(ctx, &views);
-    if (rc) return rc;
+    take_views(ctx, buf.data(), &views);
     const TableHost* t = uses_table(req->method) ? &ctx->tables[req->table].h : nullptr;
     view_info_from(views[vof[0]], *req, t, info);
   }
@@ -1605,17 +1698,22 @@ int fomo_render_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* 
   std::vector<int> vof;
   rc = enqueue_batch(ctx, reqs, nreq, d.data(), nullptr, ctx->stream, infos ? &views : nullptr, &vof, &done);
   if (rc == FOMO_OK) rc = download(pending);
+  const size_t vb = rc == FOMO_OK && infos ? views_bytes(ctx) : 0;
+  char* p_views = vb ? bounce_buffer(ctx, vb) : nullptr;
+  std::vector<char> vbuf(p_views ? 0 : vb);
+  if (!p_views) p_views = vbuf.data();
+  const cudaError_t ev = vb ? queue_views(ctx, p_views, ctx->stream) : cudaSuccess;
   // the caller's buffers must not be written after return, error or not
   const cudaError_t e1 = cudaStreamSynchronize(ctx->copy_stream);
   const cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
   if (rc) return rc;
   FOMO_CUDA(e1 != cudaSuccess ? e1 : e2, "render");
+  FOMO_CUDA(ev, "view readback");
   rc = check_device_words(ctx);
   if (rc) return rc;
   if (ctx->time_march) cudaEventElapsedTime(&ctx->last_ms, ctx->scratch.ev0, ctx->scratch.ev1);
   if (infos) {
-    rc = finish_views(ctx, &views);
-    if (rc) return rc;
+    take_views(ctx, p_views, &views);
     for (int r = 0; r < nreq; ++r) {
       const TableHost* t = uses_table(reqs[r].method) ? &ctx->tables[reqs[r].table].h : nullptr;
       view_info_from(views[vof[r]], reqs[r], t, &infos[r]);
@@ -1642,17 +1740,29 @@ int fomo_render(fomo_ctx* ctx, const fomo_request* req, float* out_cube, int32_t
   int32_t* nns[1] = {d_nn};
   rc = enqueue_batch(ctx, req, 1, outs, nns, ctx->stream, info ? &views : nullptr, &vof);
   if (rc) return rc;
-  FOMO_CUDA(cudaMemcpyAsync(out_cube, d_cube, cube_elems(*req) * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream),
+  // a small result comes back through pinned memory with the view, in copies that queue behind the
+  // render; a copy to pageable memory would be waited for one by one
+  const size_t cube_raw = cube_elems(*req) * sizeof(float), vb = info ? views_bytes(ctx) : 0;
+  char* p = bounce_buffer(ctx, cube_bytes + ((nn_bytes + 255) & ~size_t(255)) + vb);
+  char* p_nn = p ? p + cube_bytes : reinterpret_cast<char*>(out_nn_idx);
+  char* p_views = p ? p + cube_bytes + ((nn_bytes + 255) & ~size_t(255)) : (vb ? bounce_buffer(ctx, vb) : nullptr);
+  std::vector<char> vbuf(p_views ? 0 : vb);
+  if (!p_views) p_views = vbuf.data();
+  FOMO_CUDA(queue_views(ctx, p_views, ctx->stream), "view readback");
+  FOMO_CUDA(cudaMemcpyAsync(p ? p : reinterpret_cast<char*>(out_cube), d_cube, cube_raw, cudaMemcpyDeviceToHost,
+                            ctx->stream),
             "cube download");
-  if (d_nn)
-    FOMO_CUDA(cudaMemcpyAsync(out_nn_idx, d_nn, nn_bytes, cudaMemcpyDeviceToHost, ctx->stream), "index download");
+  if (d_nn) FOMO_CUDA(cudaMemcpyAsync(p_nn, d_nn, nn_bytes, cudaMemcpyDeviceToHost, ctx->stream), "index download");
   FOMO_CUDA(cudaStreamSynchronize(ctx->stream), "render");
   rc = check_device_words(ctx);
   if (rc) return rc;
+  if (p) {
+    std::memcpy(out_cube, p, cube_raw);
+    if (d_nn) std::memcpy(out_nn_idx, p_nn, nn_bytes);
+  }
   if (ctx->time_march) cudaEventElapsedTime(&ctx->last_ms, ctx->scratch.ev0, ctx->scratch.ev1);
   if (info) {
-    rc = finish_views(ctx, &views);
-    if (rc) return rc;
+    take_views(ctx, p_views, &views);
     const TableHost* t = uses_table(req->method) ? &ctx->tables[req->table].h : nullptr;
     view_info_from(views[vof[0]], *req, t, info);
   }

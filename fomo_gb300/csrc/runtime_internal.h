@@ -186,6 +186,9 @@ struct fomo_ctx {
   fomo::ScratchSet scratch;  // descriptors, per-view tables, Thomson sin^2 chi
   fomo::Arena out_arena;     // device cubes of host-output renders
   std::vector<fomo::ViewReadback> view_readback;
+  // pinned host memory for small results and scalars that are read back (kept, at most kBounceMax)
+  char* bounce = nullptr;
+  size_t bounce_cap = 0;
   double cell_occupancy = 2.0;  // target points per grid cell (FOMO_CELL_OCCUPANCY)
   bool occupancy_set = false;   // set explicitly: no per-snapshot choice (see build_snapshot)
   int64_t npos_cap = int64_t(1) << 31;  // neighbour-buffer entries per launch (FOMO_NPOS_CAP): 8 GiB
@@ -209,7 +212,8 @@ namespace fomo {
 int set_err(fomo_ctx* c, int code, const std::string& msg);
 int cuda_err(fomo_ctx* c, cudaError_t e, const char* what);
 int dev_alloc(fomo_ctx* ctx, void** p, size_t bytes);
-void dev_free(fomo_ctx* ctx, void* p);
+// idle: the device is known to be done with p (a kept block is otherwise given back after a synchronize).
+void dev_free(fomo_ctx* ctx, void* p, bool idle = false);
 void release_free_blocks(fomo_ctx* ctx);  // cudaFree of the blocks dev_free kept
 int validate(fomo_ctx* ctx, const fomo_request& q);
 size_t cube_elems(const fomo_request& q);
@@ -217,7 +221,7 @@ size_t cube_elems(const fomo_request& q);
 // stream: their cubes are complete when the stream reaches that point.  With
 // it, a launch marches in view ranges: ranges of about `range_cost` LOS
 // samples + output cells each when that is > 0, else up to 8 ranges, one per
-// 256 MB of cubes.
+// 64 MB of cubes.
 using RangeDone = std::function<int(const PlanGroup& G, int v0, int v1)>;
 int enqueue_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* d_out, int32_t* const* d_nn,
                   cudaStream_t s, std::vector<ViewDesc>* views_out, std::vector<int>* view_of_req,
@@ -232,7 +236,6 @@ SnapDev snap_dev(const SnapRec& r);
 float payload_wmax(fomo_ctx* ctx, int snap, int table, int imaging, double abund);
 void line_window(double lwa, int L, double lambda0, float vmax, float wmax, int* wstart, int* nw);
 void fill_view_host(const fomo_request& q, double lambda0, int tw, int th, ViewDesc* V);
-int finish_views(fomo_ctx* ctx, std::vector<ViewDesc>* views);
 void view_info_from(const ViewDesc& V, const fomo_request& q, const TableHost* t, fomo_view_info* info);
 int parse_table_text(const std::string& text, TableHost* t, std::string* err);
 bool parse_tune_line(const std::string& line, std::string* key, TuneChoice* c);
