@@ -79,6 +79,11 @@ namespace {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = 128;
 constexpr int kWarps = kThreads / 32;
+// Units of search work per resident warp below which rays (or blocks of rays) are cut into stretches
+// of segments: a warp that walks a whole ray of a small view is most of that view's time.  64^2 to
+// 700^2 views through four snapshots one after the other, sum of the searches: 13.9 ms as whole rays,
+// 12.4 ms at 4 units, 12.2 ms at 8; large views have units enough as whole rays.
+constexpr int kUnitsPerWarp = 8;
 constexpr int kMinCtas = 4;  // resident CTAs per SM: 16 warps of latency hiding at <= 128 registers
 constexpr int kMinCtasSearch = 7;   // the search-only pass: 28 warps at <= 72 registers (31 KB shared per CTA)
 constexpr int kMinCtasBundle = 5;   // the search over blocks of rays: 20 warps at <= 102 registers (at 64 views x 4 lines: 37.1, 35.4, 38.4, 37.7 ms at 4 to 7 CTAs)
@@ -266,10 +271,17 @@ __device__ __forceinline__ bool ray_of_item(const MarchArgs& a, const double3* k
   return true;
 }
 
-// Warp-collective: the next ray of the work queue (items item_base ..
-// end - 1, head counter `ctr`), false when the queue is drained.
-__device__ __forceinline__ bool next_ray(const MarchArgs& a, const double3* ktab, int ktab_stride, int64_t end,
-                                         RayCtx& r, int ctr = kCtrRays) {
+// Part `part` of `parts` of a ray of nz samples: samples [s0, s1), whole segments.
+__device__ __forceinline__ void part_segments(int nz, int part, int parts, int& s0, int& s1) {
+  const int nsegs = (nz + kSeg - 1) / kSeg;
+  s0 = (int)((int64_t)nsegs * part / parts) * kSeg;
+  s1 = min((int)((int64_t)nsegs * (part + 1) / parts) * kSeg, nz);
+}
+
+// Warp-collective: the next unit of the work queue (items item_base ..
+// end - 1 in `parts` parts each, head counter `ctr`), false when the queue is drained.
+__device__ __forceinline__ bool next_part(const MarchArgs& a, const double3* ktab, int ktab_stride, int64_t end,
+                                          int parts, RayCtx& r, int& part, int ctr = kCtrRays) {
   const int lane = threadIdx.x & 31;
   for (;;) {
     unsigned long long item = 0;
@@ -279,12 +291,25 @@ __device__ __forceinline__ bool next_ray(const MarchArgs& a, const double3* ktab
       // drained.  The word only goes from 0 to 1 while a batch runs, so a
       // kernel that starts after one that stopped stops at its first ray too
       // (an emission pass reads no position its search did not write).
-      if (a.stop && __ldcv(a.stop) != 0u) item = (unsigned long long)end;
+      if (a.stop && __ldcv(a.stop) != 0u) item = (unsigned long long)end * (unsigned)parts;
     }
-    item = __shfl_sync(kFull, item, 0) + (unsigned long long)a.item_base;
+    item = __shfl_sync(kFull, item, 0);
+    part = 0;
+    if (parts > 1) {
+      const unsigned long long unit = item;
+      item = unit / (unsigned)parts;
+      part = (int)(unit - item * (unsigned)parts);
+    }
+    item += (unsigned long long)a.item_base;
     if ((int64_t)item >= end) return false;
     if (ray_of_item(a, ktab, ktab_stride, (int64_t)item, r)) return true;
   }
+}
+// ..whole rays
+__device__ __forceinline__ bool next_ray(const MarchArgs& a, const double3* ktab, int ktab_stride, int64_t end,
+                                         RayCtx& r, int ctr = kCtrRays) {
+  int part;
+  return next_part(a, ktab, ktab_stride, end, 1, r, part, ctr);
 }
 
 // LOS sample k: derotated position (nn:162-165) in FP64.
@@ -479,24 +504,30 @@ __device__ __forceinline__ PartOut segment_parts(const MarchArgs& a, const RayCt
           const int excl = incl - n;
           const int total = __shfl_sync(kFull, incl, 31);
           st_loaded += total;
-          for (int ib = 0; ib < total; ib += 32) {
-            const int i = ib + lane;
-            const int own = warp_owner(incl, i);
-            const int ob = __shfl_sync(kFull, base, own);
-            const int oe = __shfl_sync(kFull, excl, own);
-            bool keep = false;
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            int p = 0, bk = 0;
-            if (i < total) {
-              p = ob + (i - oe);
-              q = __ldg(S.pts + FOMO_IDX(p, S.n, kSitePts));
-              const float wx = q.x - ax, wy = q.y - ay, wz = q.z - az;
-              float s = fmaf(wz, sdz, fmaf(wy, sdy, wx * sdx)) * inv_len2;
-              s = fminf(fmaxf(s, 0.0f), 1.0f);
-              const float ex = fmaf(-s, sdx, wx), ey = fmaf(-s, sdy, wy), ez = fmaf(-s, sdz, wz);
-              keep = fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= Rg2;
-              bk = min(max(__float2int_rn(s * (float)(pn - 1)), 0), pn - 1);
+          float4 qn = make_float4(0.f, 0.f, 0.f, 0.f);
+          int pt = 0;
+          // the next 32 points are loaded before these are tested; a list that overflowed stops
+          for (int ib = 0; ib < total + 32 && count <= kSegCap; ib += 32) {
+            const float4 q = qn;
+            const int p = pt;
+            const bool have = ib > 0 && ib - 32 + lane < total;
+            if (ib < total) {
+              const int i = ib + lane;
+              const int own = warp_owner(incl, i);
+              const int ob = __shfl_sync(kFull, base, own);
+              const int oe = __shfl_sync(kFull, excl, own);
+              if (i < total) {
+                pt = ob + (i - oe);
+                qn = __ldg(S.pts + FOMO_IDX(pt, S.n, kSitePts));
+              }
             }
+            if (ib == 0) continue;
+            const float wx = q.x - ax, wy = q.y - ay, wz = q.z - az;
+            float s = fmaf(wz, sdz, fmaf(wy, sdy, wx * sdx)) * inv_len2;
+            s = fminf(fmaxf(s, 0.0f), 1.0f);
+            const float ex = fmaf(-s, sdx, wx), ey = fmaf(-s, sdy, wy), ez = fmaf(-s, sdz, wz);
+            const bool keep = have && fmaf(ez, ez, fmaf(ey, ey, ex * ex)) <= Rg2;
+            const int bk = min(max(__float2int_rn(s * (float)(pn - 1)), 0), pn - 1);
             const unsigned msk = __ballot_sync(kFull, keep);
             if (keep) {
               const int slot = count + __popc(msk & lt);
@@ -757,7 +788,7 @@ __device__ __forceinline__ void segment_search(const MarchArgs& a, const RayCtx&
         const int excl = incl - n;
         const int total = __shfl_sync(kFull, incl, 31);
         st_loaded += total;
-        for (int ib = 0; ib < total; ib += 32) {
+        for (int ib = 0; ib < total && count <= kSegCap; ib += 32) {
           const int i = ib + lane;
           const int own = warp_owner(incl, i);
           const int ob = __shfl_sync(kFull, base, own);
@@ -976,13 +1007,16 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSearch) march_search(MarchAr
   SegSmem& sm = segs[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   RayCtx r;
-  while (next_ray(a, ktab, ktab_stride, min(a.total_items, a.bundle_from), r)) {
+  int part;
+  while (next_part(a, ktab, ktab_stride, min(a.total_items, a.bundle_from), a.parts, r, part)) {
     const ViewDesc* V = a.views + r.v;
     const int nz = V->nz;
     int32_t* nnout = a.nn_idx ? a.nn_idx[r.v] : nullptr;
     const int64_t ray = (int64_t)r.i * V->nx + r.j;
     int32_t* npos = a.npos + ((int64_t)r.item - a.item_base) * ktab_stride;
-    for (int s0 = 0; s0 < nz; s0 += kSeg) {
+    int s0, s1;
+    part_segments(nz, part, a.parts, s0, s1);
+    for (; s0 < s1; s0 += kSeg) {
       int posv[2], origv[2];
       segment_search(a, r, s0, nz, sm, posv, origv);
 #pragma unroll
@@ -2402,9 +2436,13 @@ __device__ __forceinline__ void store_deferred(const MarchArgs& a, const RayCtx&
 // (dense clumps, long segments at a coarse LOS step) is queued by the first
 // pass at the back of the deferred buffer with all its samples.  This kernel
 // searches each such segment again as parts of 32 samples (16 when a part
-// overflows too), each part gathering its own, shorter capsule, stores the
+// overflows too), a warp per part, each part gathering its own, shorter capsule, stores the
 // neighbours of the samples it resolves (POS) or adds their emission, and
 // rewrites the record with the samples still unresolved, for march_deferred.
+// What bounds it is one warp's chain of loads: the overflowing segments of a 96^2 to 700^2 view
+// are few and their capsules hold hundreds of points.  One after the other, 20 views of
+// 64^2 to 700^2: 6.1 ms; 4.9 ms when a full list stops the gather within its rows;
+// 3.9 ms with a warp per half; 3.4 ms with a round of points loaded ahead.
 // ---------------------------------------------------------------------------
 template <bool POS>
 __global__ void __launch_bounds__(kThreads, kMinCtasSplit) march_split(MarchArgs a, const double3* __restrict__ ktab,
@@ -2420,18 +2458,21 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSplit) march_split(MarchArgs
     unsigned long long k = 0;
     if (lane == 0) k = atomicAdd(a.counter + kCtrOverflowHead, 1ull);
     k = __shfl_sync(kFull, k, 0);
-    if ((int64_t)k >= nover) return;
-    const int64_t slot = a.deferred_cap - 1 - (int64_t)k;
-    const DeferredRec rec = a.deferred[FOMO_IDX(slot, a.deferred_cap, kSiteDeferred)];
+    if ((int64_t)k >= 2 * nover) return;
+    const int half = (int)(k & 1);  // the two warps of a record write a word each, and read their own
+    const int64_t slot = a.deferred_cap - 1 - (int64_t)(k >> 1);
+    DeferredRec* rec = a.deferred + FOMO_IDX(slot, a.deferred_cap, kSiteDeferred);
+    unsigned* open = half ? &rec->w : &rec->z;
+    const unsigned item = rec->x, mask = *open;
     RayCtx r;
-    if (!ray_of_item(a, ktab, ktab_stride, (int64_t)rec.x, r)) continue;  // records come from real rays only
+    if (!ray_of_item(a, ktab, ktab_stride, (int64_t)item, r)) continue;  // records come from real rays only
     const ViewDesc* V = a.views + r.v;
-    const int nz = V->nz, s0 = (int)(rec.y & kRecS0);
+    const int nz = V->nz, s0 = (int)(rec->y & kRecS0);
     PartIn in;
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int kk = s0 + lane + 32 * i;
-      in.act[i] = kk < nz && (((i ? rec.w : rec.z) >> lane) & 1u);
+      in.act[i] = kk < nz && i == half && ((mask >> lane) & 1u);
       double p0 = 0.0, p1 = 0.0, p2 = 0.0;
       if (kk < nz) sample_pos(r, kk, p0, p1, p2);
       in.tx[i] = __double2float_rn(p0);  // the FP32 target (nn:171)
@@ -2448,7 +2489,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSplit) march_split(MarchArgs
       const bool done = in.act[i] && !o.need[i];
       if (nnout && done) nnout[FOMO_IDX(ray * nz + s0 + lane + 32 * i, (int64_t)V->nx * V->ny * nz, kSiteNnIdx)] = o.orig[i];
       if (POS) {
-        if (done) *npos_at(a, rec.x, s0 + lane + 32 * i, ktab_stride) = o.pos[i];
+        if (done) *npos_at(a, item, s0 + lane + 32 * i, ktab_stride) = o.pos[i];
         continue;
       }
       const bool fill = done && o.pos[i] >= 0;
@@ -2472,7 +2513,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSplit) march_split(MarchArgs
     }
     const unsigned f0 = __ballot_sync(kFull, in.act[0] && o.need[0]);
     const unsigned f1 = __ballot_sync(kFull, in.act[1] && o.need[1]);
-    if (lane == 0) a.deferred[FOMO_IDX(slot, a.deferred_cap, kSiteDeferred)] = make_uint4(rec.x, rec.y, f0, f1);
+    if (lane == 0) *open = half ? f1 : f0;
   }
 }
 
@@ -3030,7 +3071,12 @@ cudaError_t launch_march(const MarchArgs& a, const double3* ktab, int ktab_strid
     e = cudaSuccess;
     const int64_t single = std::min(a.total_items, a.bundle_from) - a.item_base;
     const int64_t bundles = (a.total_items - std::max(a.item_base, a.bundle_from)) / 4;
-    if (single > 0) e = launch_persistent(march_search, a, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint, single);
+    if (single > 0) {
+      MarchArgs b = a;
+      const int64_t want = kUnitsPerWarp * (int64_t)sm_count * kMinCtasSearch * kWarps;
+      b.parts = (int)std::max<int64_t>(1, std::min<int64_t>((want + single - 1) / single, (ktab_stride + kSeg - 1) / kSeg));
+      e = launch_persistent(march_search, b, ktab, ktab_stride, sm_count, s, blocks_per_sm_hint, single * b.parts);
+    }
     if (e == cudaSuccess && bundles > 0) {
       // a unit is a stretch of a bundle's segments: all of them where there are
       // bundles enough for four units per warp of the GPU, single segments at the least
