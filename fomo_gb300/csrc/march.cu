@@ -2533,9 +2533,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSplit) march_split(MarchArgs
 // equator): each one's own ring walk would scan every cell of the lens where
 // the ball of its neighbour's distance cuts into the cloud, and consecutive
 // samples scan almost the same lens.  Here each pending sample gets a ball --
-// at first its distance to the points' bounding box plus three cells -- and
-// each lane marks, in shared memory, the x range its ball covers in every row
-// of cells it reaches; the warp then gathers those rows (the union of the
+// at first its distance to the points' bounding box plus three cells -- and of the rows of
+// cells that the balls reach, those that hold a point in the balls' x range are cut to the x
+// range that some ball covers there (a lane per ball, a minimum and a maximum over the warp a
+// row); the warp then gathers those rows (the union of the
 // balls), testing each gathered point against every sample's box as the
 // one-lane search does.  A sample whose best point lies
 // inside its own ball (gathered whole), without a near-tie, has its neighbour;
@@ -2543,22 +2544,34 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSplit) march_split(MarchArgs
 // when they found none, and the warp gathers again.  Samples still open after
 // kFarIters gathers, near-ties and gathers beyond the row or point bounds go
 // on to march_deferred as before.
+//
+// What bounds it is instruction issue (81 %): 1.6 gathers a half, each of 48 rows, 14 of them with points, and 39
+// points.  8M-point rope, 1024^2 Thomson view of 1024 samples: 83.3 ms with the balls' rows marked in shared memory
+// with atomics (4,200 instructions a gather), 63.4 with a reduction a row, 62.0 without branches in the point test
+// (31 -> 25 us for 45 halves) at eight CTAs, 47.9 without the empty rows (0.5M-point rope, 96^2: 230 -> 158 us).
 // ---------------------------------------------------------------------------
-constexpr int kMinCtasFar = 6;   // 24 warps per SM at <= 80 registers
+constexpr int kMinCtasFar = 8;   // 32 warps per SM at <= 64 registers (6 to 8 CTAs: 49.3, 48.5, 47.9 ms)
 constexpr int kFarRowCap = 256;  // rows of a gather's bounding rectangle (beyond: the half is left)
 struct __align__(16) FarSmem {
-  float4 pt[32];           // a round of gathered points
-  int pp[32];              // their sorted positions
-  int xlo[kFarRowCap];     // per row of the rectangle: the union of the balls' chords, as ordered ints
-  int xhi[kFarRowCap];
+  float4 pt[32];  // a round of gathered points, and their sorted positions
 };
 
-// float -> int with the same order (atomicMin / atomicMax on floats)
-__device__ __forceinline__ int ford(float f) {
-  const int i = __float_as_int(f);
-  return i >= 0 ? i : i ^ 0x7fffffff;
+__device__ __forceinline__ float rsqrt_approx(float v) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
 }
-__device__ __forceinline__ float fdeord(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+// Minimum and maximum over the warp, in one instruction each.
+__device__ __forceinline__ float redux_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float redux_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
 
 // Warp-collective search of the lanes' samples (act: this lane holds one, box
 // q).  Returns the lanes whose neighbour was found: pos / orig set, -1 when
@@ -2589,30 +2602,36 @@ __device__ __forceinline__ unsigned far_half(const SnapDev& S, const BoxQ& q, bo
   for (int it = 0; it < kFarIters && pend; ++it) {
     const bool mine = (pend >> lane) & 1u;
     float best = FLT_MAX, second = FLT_MAX;
-    int bpos = -1, borig = -1;
+    int bpos = -1;
     // the rows this lane's ball reaches, within the box: a point of the grid
     // lies at least the target's distance to the points' bounding box away
     // along each axis, so the ball's y extent there is sqrt(r^2 - dx^2 - dz^2)
     // and its z extent sqrt(r^2 - dx^2 - dy^2), dx, dy, dz those distances
-    float ylo = FLT_MAX, yhi = -FLT_MAX, zlo = FLT_MAX, zhi = -FLT_MAX;
+    float xl = FLT_MAX, xh = -FLT_MAX, ylo = FLT_MAX, yhi = -FLT_MAX, zlo = FLT_MAX, zhi = -FLT_MAX;
     if (mine) {
-      const float ry2 = r2 - fmaf(dzg, dzg, dxg * dxg), rz2 = r2 - fmaf(dyg, dyg, dxg * dxg);
-      if (ry2 >= 0.0f && rz2 >= 0.0f) {
+      const float rx2 = r2 - fmaf(dzg, dzg, dyg * dyg), ry2 = r2 - fmaf(dzg, dzg, dxg * dxg),
+                  rz2 = r2 - fmaf(dyg, dyg, dxg * dxg);
+      if (rx2 >= 0.0f && ry2 >= 0.0f && rz2 >= 0.0f) {
+        const float rx = (rx2 > 0.0f ? rx2 * rsqrtf(rx2) * 1.0001f : 0.0f) + kCellMargin * h;
         const float ry = (ry2 > 0.0f ? ry2 * rsqrtf(ry2) * 1.0001f : 0.0f) + kCellMargin * h;
         const float rz = (rz2 > 0.0f ? rz2 * rsqrtf(rz2) * 1.0001f : 0.0f) + kCellMargin * h;
+        xl = fmaxf(q.tx - rx, q.lox);
+        xh = fminf(q.tx + rx, q.hix);
         ylo = fmaxf(q.ty - ry, q.loy);
         yhi = fminf(q.ty + ry, q.hiy);
         zlo = fmaxf(q.tz - rz, q.loz);
         zhi = fminf(q.tz + rz, q.hiz);
       }
     }
-    ylo = warp_min(ylo);
-    yhi = warp_max(yhi);
-    zlo = warp_min(zlo);
-    zhi = warp_max(zhi);
+    xl = redux_min(xl);
+    xh = redux_max(xh);
+    ylo = redux_min(ylo);
+    yhi = redux_max(yhi);
+    zlo = redux_min(zlo);
+    zhi = redux_max(zhi);
     bool overflow = false;
     int j0 = 0, k0 = 0, nyr = 0, nrows = 0;
-    if (ylo <= yhi && zlo <= zhi) {
+    if (xl <= xh && ylo <= yhi && zlo <= zhi) {
       j0 = cell_coord(ylo, g.oy, g.inv_h, g.dy);
       const int j1 = cell_coord(yhi, g.oy, g.inv_h, g.dy);
       k0 = cell_coord(zlo, g.oz, g.inv_h, g.dz);
@@ -2620,54 +2639,47 @@ __device__ __forceinline__ unsigned far_half(const SnapDev& S, const BoxQ& q, bo
       nyr = j1 - j0 + 1;
       nrows = nyr * (k1 - k0 + 1);
       overflow = nrows > kFarRowCap;
-      if (!overflow) {
-        for (int i = lane; i < nrows; i += 32) {
-          fs.xlo[i] = ford(FLT_MAX);
-          fs.xhi[i] = ford(-FLT_MAX);
-        }
-        __syncwarp();
-        if (mine) {
-          // this lane's rows: where its ball reaches the grid's x range, in the rectangle
-          const float rx2 = r2 - dxg * dxg;
-          int z0 = k0, z1 = k1;
-          clip_reach(rx2 - dyg * dyg, q.tz, g.oz, g.inv_h, h, g.dz, z0, z1);
-          for (int kz = z0; kz <= z1; ++kz) {
-            const float gz = axis_gap(kz, q.tz, g.oz, h);
-            const float gz2 = gz * gz;
-            int y0 = j0, y1 = j0 + nyr - 1;
-            clip_reach(rx2 - gz2, q.ty, g.oy, g.inv_h, h, g.dy, y0, y1);
-            for (int jy = y0; jy <= y1; ++jy) {
-              const float gy = axis_gap(jy, q.ty, g.oy, h);
-              const float rem = r2 - fmaf(gy, gy, gz2);
-              if (rem >= 0.0f) {
-                const float rx = (rem > 0.0f ? rem * rsqrtf(rem) * 1.0001f : 0.0f) + kCellMargin * h;
-                const float xa = fmaxf(q.tx - rx, q.lox), xb = fminf(q.tx + rx, q.hix);
-                if (xa <= xb) {
-                  const int row = (kz - k0) * nyr + (jy - j0);
-                  atomicMin(&fs.xlo[row], ford(xa));
-                  atomicMax(&fs.xhi[row], ford(xb));
-                }
-              }
-            }
-          }
-        }
-        __syncwarp();
-      }
       int npts = 0;
       const float inv_nyr = nyr > 0 ? 1.0f / (float)nyr : 0.0f;
+      // distances of the target from the middle of row j0 + y of layer k0 + z: |ey - y h|, |ez - z h|; up to
+      // wy, wz (half a cell, its margin and the rounding of the coordinates) the target lies in the row's slab
+      const float mr2 = mine ? r2 : -1.0f;
+      const float ey = q.ty - fmaf((float)j0 + 0.5f, h, g.oy), ez = q.tz - fmaf((float)k0 + 0.5f, h, g.oz);
+      const float wy = (0.5f + kCellMargin) * h + (fabsf(q.ty) + fabsf(g.oy)) * 4.8e-7f;
+      const float wz = (0.5f + kCellMargin) * h + (fabsf(q.tz) + fabsf(g.oz)) * 4.8e-7f;
+      const int xc0 = cell_coord(xl, g.ox, g.inv_h, g.dx), xc1 = cell_coord(xh, g.ox, g.inv_h, g.dx);
       for (int rb = 0; rb < nrows && !overflow; rb += 32) {
-        const int rr = rb + lane;
-        int base = 0, n = 0;
-        if (rr < nrows) {
-          int ry;
-          const int kz = k0 + row_div(rr, nyr, inv_nyr, ry), jy = j0 + ry;
-          const float xa = fdeord(fs.xlo[rr]), xb = fdeord(fs.xhi[rr]);
-          if (xa <= xb && xb >= g.minx && xa <= g.maxx) {
-            const int c0 = cell_coord(xa, g.ox, g.inv_h, g.dx), c1 = cell_coord(xb, g.ox, g.inv_h, g.dx);
-            const int rowbase = (kz * g.dy + jy) * g.dx;
-            base = __ldg(S.cell_start + FOMO_IDX(rowbase + c0, cell_entries(g), kSiteCellStart));
-            n = __ldg(S.cell_start + FOMO_IDX(rowbase + c1 + 1, cell_entries(g), kSiteCellStart)) - base;
+        // a row per lane; most hold no point in the x range of the balls (beside a rope of points, 33 of 48)
+        int rowbase = 0, ry = 0, rz = 0;
+        bool row = rb + lane < nrows;
+        if (row) {
+          rz = row_div(rb + lane, nyr, inv_nyr, ry);
+          rowbase = ((k0 + rz) * g.dy + j0 + ry) * g.dx;
+          row = __ldg(S.cell_start + FOMO_IDX(rowbase + xc0, cell_entries(g), kSiteCellStart)) !=
+                __ldg(S.cell_start + FOMO_IDX(rowbase + xc1 + 1, cell_entries(g), kSiteCellStart));
+        }
+        const float fy = (float)ry, fz = (float)rz;
+        // the union of the balls' chords in each of the others, lane t's in row rb + t
+        float xlo = FLT_MAX, xhi = -FLT_MAX;
+        for (unsigned todo = __ballot_sync(kFull, row); todo; todo &= todo - 1u) {
+          const int t = __ffs(todo) - 1;
+          const float gy = fmaxf(fabsf(fmaf(-__shfl_sync(kFull, fy, t), h, ey)) - wy, 0.0f);
+          const float gz = fmaxf(fabsf(fmaf(-__shfl_sync(kFull, fz, t), h, ez)) - wz, 0.0f);
+          const float rem = fmaf(-gy, gy, fmaf(-gz, gz, mr2)), rp = fmaxf(rem, 1e-35f);
+          const float rx = fmaf(rp * rsqrt_approx(rp), 1.0001f, kCellMargin * h);
+          const float xa = fmaxf(q.tx - rx, q.lox), xb = fminf(q.tx + rx, q.hix);
+          const bool on = rem >= 0.0f && xa <= xb;
+          const float lo = redux_min(on ? xa : FLT_MAX), hi = redux_max(on ? xb : -FLT_MAX);
+          if (lane == t) {
+            xlo = lo;
+            xhi = hi;
           }
+        }
+        int base = 0, n = 0;
+        if (xlo <= xhi && xhi >= g.minx && xlo <= g.maxx) {
+          const int c0 = cell_coord(xlo, g.ox, g.inv_h, g.dx), c1 = cell_coord(xhi, g.ox, g.inv_h, g.dx);
+          base = __ldg(S.cell_start + FOMO_IDX(rowbase + c0, cell_entries(g), kSiteCellStart));
+          n = __ldg(S.cell_start + FOMO_IDX(rowbase + c1 + 1, cell_entries(g), kSiteCellStart)) - base;
         }
         // the rows' points, 32 per round, each tested by every pending lane
         const int incl = warp_incl_scan(n);
@@ -2684,31 +2696,25 @@ __device__ __forceinline__ unsigned far_half(const SnapDev& S, const BoxQ& q, bo
           const int ob = __shfl_sync(kFull, base, own), oe = __shfl_sync(kFull, excl, own);
           if (i < total) {
             const int p = ob + (i - oe);
-            fs.pt[lane] = __ldg(S.pts + FOMO_IDX(p, S.n, kSitePts));
-            fs.pp[lane] = p;
+            float4 v = __ldg(S.pts + FOMO_IDX(p, S.n, kSitePts));
+            v.w = __int_as_float(p);
+            fs.pt[lane] = v;
           }
           __syncwarp();
           const int cn = min(32, total - ib);
           if (mine) {
-            // every point of the round against this lane's best and box (the
-            // same test as scan_point); four at a time, their distances independent
+            // every point of the round against this lane's box and best; without branches: a
+            // point is nearer than some lane's second best about every time
 #pragma unroll 4
             for (int k = 0; k < cn; ++k) {
               const float4 v = fs.pt[k];
               const float dx = v.x - q.tx, dy = v.y - q.ty, dz = v.z - q.tz;
-              const float d = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-              // rare once the lane has two in-box points: kept a branch around the box test
-              if (__builtin_expect(d < second, 0)) {
-                if (v.x > q.lox && v.x < q.hix && v.y > q.loy && v.y < q.hiy && v.z > q.loz && v.z < q.hiz) {
-                  if (d < best) {
-                    second = best;
-                    best = d;
-                    bpos = fs.pp[k];
-                    borig = __float_as_int(v.w);
-                  } else {
-                    second = d;
-                  }
-                }
+              const bool in = (v.x > q.lox) & (v.x < q.hix) & (v.y > q.loy) & (v.y < q.hiy) & (v.z > q.loz) & (v.z < q.hiz);
+              const float d = in ? fmaf(dz, dz, fmaf(dy, dy, dx * dx)) : FLT_MAX;
+              second = fminf(second, fmaxf(best, d));
+              if (d < best) {
+                best = d;
+                bpos = __float_as_int(v.w);
               }
             }
           }
@@ -2723,7 +2729,7 @@ __device__ __forceinline__ unsigned far_half(const SnapDev& S, const BoxQ& q, bo
     const bool tie = found && second <= best * (1.0f + kRelTie);
     if (found && !tie) {
       pos = bpos;
-      orig = borig;
+      orig = __float_as_int(__ldg(&S.pts[FOMO_IDX(bpos, S.n, kSitePts)].w));
     }
     solved |= __ballot_sync(kFull, found && !tie);
     margin2 *= 4.0f;
