@@ -126,7 +126,7 @@ struct MarchArgs {
   const float2* ktf;             // per view and LOS sample: the LOS table's x, -y, z as FP32 pairs (high, low part)
   int64_t bundle_from;           // work items from here on are searched as 2 x 2 blocks of rays (a multiple of 4)
   int parts;                     // work units per block of rays: stretches of its segments
-  float rscale;                  // gather radius of the search in local point spacings (0: the default, 0.9)
+  float rscale;                  // gather radius of the search in local point spacings
   unsigned long long* stats;     // optional search counters (profiling), else null
   const unsigned* stop;          // a server batch's stop word (device memory), or null: once it is
                                  // set, the ray-queue kernels take no further rays

@@ -97,7 +97,6 @@ constexpr float kCellMargin = 0.02f;  // cell-boundary slack in cells (binning e
 constexpr int kSeg = 64;              // LOS samples per segment (two per lane)
 constexpr int kSegCap = 176;          // candidates per segment (sized so that 7 search CTAs fit an SM)
 constexpr int kMaxRows = 4096;        // cell rows of a segment's capsule beyond which it is deferred
-constexpr float kRScaleDefault = 0.9f;  // gather radius in local point spacings (MarchArgs::rscale when set)
 // Far pass (march_far): samples half a cell or more off the points' bounding box,
 // kFarMin or more of them in a half record, searched together by a warp.
 constexpr int kFarMin = 4;          // far samples a half needs (fewer: the lane walks of march_deferred)
@@ -385,7 +384,7 @@ __device__ __forceinline__ void clip_interval(float a, float d, float inv_d, flo
 __device__ __forceinline__ float gather_radius(const MarchArgs& a, float mdf, float aloc, float amax) {
   const float md_seg = mdf + (amax + mdf) * 4.8e-7f + mdf * 1.2e-7f;
   const float cap = fmaf(md_seg * 1.7321f, 1.0001f, amax * 4.8e-7f) * 1.0001f;
-  return fminf(cap, (a.rscale > 0.0f ? a.rscale : kRScaleDefault) * aloc);
+  return fminf(cap, a.rscale * aloc);
 }
 
 struct PartIn {

@@ -840,6 +840,14 @@ bool bundle_view(const SnapRec& snap, const fomo_request& q, int tw, int th, boo
   return view_pitch(snap, q) <= (snap.uniform ? kBundlePitch : kBundlePitchClustered) * snap.spacing;
 }
 
+// The search's gather radius in local point spacings (a sample whose neighbour is farther goes to the deferred passes).
+// A wider one gathers more points per segment, a narrower one leaves more samples to the
+// lane walks, which cost most in a clustered cloud.  All march kernels at 0.8 / 0.87 / 0.9 / 1.0 / 1.1:
+// 2M-point loop, 64 views 58.2 / 58.4 / 58.9 / 61.5 / 65.0 ms; 262K points, 256^2 x 256 731 / 736 / 747 / 879 / 893 us;
+// 40K points, 149 x 100 x 300 pixels 271 / 264 / 272 / 262 / 277 us; clustered: 8M-point rope, 1024^3
+// 23.9 / - / 22.2 / 21.4 / 20.9 ms (1.25: 21.6), its Thomson view - / - / 103.5 / 101.4 / 98.9 ms.
+constexpr float kRadiusUniform = 0.87f, kRadiusClustered = 1.1f;
+
 // Plan a batch.  Requests are grouped into launches by (snapshot, method,
 // imaging); inside a launch, requests with the same view (angles, resolution,
 // width) become lines of one view and share the neighbour search.  All
@@ -950,6 +958,7 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     G.th = ctx->tile_h;
     G.bps = ctx->blocks_per_sm;
     G.rscale = ctx->rscale;
+    G.uniform = snap.uniform;
     if (G.tw <= 0 || G.th <= 0) {
       G.tw = 8;
       G.th = 4;
@@ -1210,7 +1219,7 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
     a.s2 = s2;
     a.totpol = G.totpol;
     a.stats = ctx->march_stats;
-    a.rscale = G.rscale;
+    a.rscale = G.rscale > 0.0f ? G.rscale : (G.uniform ? kRadiusUniform : kRadiusClustered);
     a.stop = scr->stop;
     if (e == cudaSuccess && scr->ev0 && ctx->time_march) e = record_timing(scr->ev0);
     MarchTimer* timer = (ctx->kernel_timing && !capturing) ? &ctx->timer : nullptr;

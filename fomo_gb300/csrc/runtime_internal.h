@@ -109,6 +109,7 @@ struct PlanGroup {
   int max_nw = 1;  // largest number of 32-bin lambda windows of a line
   int tw = 8, th = 4, bps = 0;
   float rscale = 0.0f;
+  bool uniform = false;  // the snapshot's points are close to uniform at the cell scale
   std::vector<const float2*> ew;       // payload per request (NN)
   const float2* totpol = nullptr;      // Thomson payload
   bool any_nn = false;
