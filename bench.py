@@ -140,13 +140,13 @@ def make_workload(seed=1):
 def kernel_bounds(kernel_ms, counters, ceilings, clocks, samples):
     """Each march kernel of the batch against the ceiling that binds it.
 
-    march_search: instruction issue -- warp instructions per LOS sample (the
+    Search: instruction issue -- warp instructions per LOS sample (the
     committed ncu figure, profiles/march_ceilings.json) x samples / its time,
     against 4 warp instructions per clock per SM at the sampled SM clock; and
     its point loads (16 B each, counted) against the measured L2 gather rate.
     Emission pass: the same issue figure, and its ex2 evaluations (counted) /
-    its time against the measured SFU throughput; it waits on its payload
-    gathers, below both.  Deferred / split / hard: their time and share."""
+    its time against the measured SFU throughput.  Deferred / split / hard:
+    their time and share."""
     total = sum(kernel_ms.values()) or 1.0
     mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 2070.0
     issue_peak = 4.0 * ceilings["sm_count"] * mhz * 1e6  # warp instructions per second
@@ -184,7 +184,7 @@ def kernel_bounds(kernel_ms, counters, ceilings, clocks, samples):
             rate = counters["ex2"] / sec
             e["sfu"] = {"achieved": rate, "peak": ceilings["ex2_per_s"], "frac": rate / ceilings["ex2_per_s"],
                         "unit": "ex2/s", "runs": counters.get("runs")}
-        e["bound"] = "latency (payload gathers per run)"
+        e["bound"] = "issue (and L1: payload gathers per run)"
     for k in ("deferred", "split", "hard"):
         if k in out:
             out[k]["bound"] = "latency (dependent L2 loads per ring)"
@@ -570,11 +570,10 @@ def run_ours(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_source": f"{peak_kind} hbm_gbs",
                          "bytes_per_sample": bps,
-                         "kernel": "march_search (neighbour search, positions to a buffer) + march_split "
-                                   "(overflowing segments) + march_far (far samples of wide-box views; an empty "
-                                   "list here) + march_deferred (the samples the search leaves) + "
-                                   "march_hard (deferred samples over the one-lane budget) + "
-                                   "march_shade_spectral<4,1> (emission from the positions), timed together",
+                         "kernel": "march_search_bundle (neighbour search over 2 x 2 blocks of rays, positions to a "
+                                   "buffer) + march_split (overflowing segments) + march_deferred (the samples "
+                                   "the search leaves) + march_shade_spectral<4,1> (emission from the "
+                                   "positions), timed together",
                          "binding": binding_bound(kernels)},
             "cpu_baseline": cpu,
             "autotuned": tuned,

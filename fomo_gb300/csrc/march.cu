@@ -2,7 +2,8 @@
 // fomo-thomson.cpp:268-343), one warp per ray, persistent over a queue of
 // (view, ray) work items so that many views and requests share one launch.
 //
-// Kernels, in stream order: march_search (stores each sample's neighbour in a
+// Kernels, in stream order: march_search and march_search_bundle (one ray, or a block of 2 x 2
+// rays, per warp; store each sample's neighbour in a
 // position buffer), march_split (segments whose capsule overflowed),
 // march_far (deferred samples far off the points, searched together),
 // march_deferred (the other samples the search could not resolve, one lane
@@ -52,12 +53,12 @@
 // Either way the chosen neighbour is the FP64 argmin strictly inside the box.
 //
 // Spectroscopic mode: equal neighbours of consecutive samples are merged into
-// runs (warp ballot); the lane starting a run loads its payload and forms, per
-// line, count * eps, 2 / w and the Doppler term; every lane then adds
+// runs (warp ballot), gathered 32 at a time; a lane loads a run's payload and forms, per
+// line, count * eps, 2 / w and the Doppler term; the lanes then add
 // count * eps * 2^(-(2 (lambda - shift) / w)^2)  (= eps exp(-4 ln2 (dl/w)^2),
-// nn:204) to its lambda bins of the line's window (the bins where any point's
-// Gaussian can exceed 2^-64 of its peak; the others are written as 0) in a
-// per-chunk FP32 partial, folded into the per-ray sum with Kahan compensation.
+// nn:204) to their lambda bins of the line's window (the bins where any point's
+// Gaussian can exceed 2^-64 of its peak; the others are written as 0) in
+// FP32 partials, folded into the per-ray sum with Kahan compensation.
 // Imaging (L = 1) and Thomson (pB) add per-sample values through a warp
 // reduction.  One warp owns one ray in the emission pass, which sums its
 // samples in order (no atomics), so a cube does not depend on what else
