@@ -85,6 +85,7 @@ constexpr int kWarps = kThreads / 32;
 // 700^2 views through four snapshots one after the other, sum of the searches: 13.9 ms as whole rays,
 // 12.4 ms at 4 units, 12.2 ms at 8; large views have units enough as whole rays.
 constexpr int kUnitsPerWarp = 8;
+constexpr int kMinCtasHard = 8;     // whole-warp walks: 32 warps at 64 registers (96^2 view of the 0.5M-point rope 101, 90, 85 us at 4, 6, 8 CTAs)
 constexpr int kMinCtas = 4;  // resident CTAs per SM: 16 warps of latency hiding at <= 128 registers
 constexpr int kMinCtasSearch = 7;   // the search-only pass: 28 warps at <= 72 registers (31 KB shared per CTA)
 constexpr int kMinCtasBundle = 5;   // the search over blocks of rays: 20 warps at <= 102 registers (at 64 views x 4 lines: 37.1, 35.4, 38.4, 37.7 ms at 4 to 7 CTAs)
@@ -2139,7 +2140,10 @@ __device__ __forceinline__ bool box_cells(const GridParams& g, const BoxQ& q, in
   return true;
 }
 
-constexpr int kLaneBudget = 192;  // rows + points one lane may scan for one sample
+// Rows + points one lane may scan for one sample before a warp takes it.  Deferred / hard pass at 192, 128, 96, 64: 24 views
+// of 64^2 to 700^2 pixels one after the other 7.7 / 2.35, 7.2 / 2.40, 7.0 / 2.44, 6.5 / 2.68 ms (the longest walk is the deferred pass's
+// time there); with range bounds of 32 and 24 points in place of kLaneDense no better.
+constexpr int kLaneBudget = 64;
 
 // Nearest point strictly inside box q, searched by this lane alone: sorted
 // position and original index, or -1 when the box holds no point.  With
@@ -2939,7 +2943,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasDeferred) march_deferred(Mar
 // emission with atomics.
 // ---------------------------------------------------------------------------
 template <bool POS>
-__global__ void __launch_bounds__(kThreads, kMinCtas) march_hard(MarchArgs a, const double3* __restrict__ ktab,
+__global__ void __launch_bounds__(kThreads, kMinCtasHard) march_hard(MarchArgs a, const double3* __restrict__ ktab,
                                                        int ktab_stride, int kind) {
   __shared__ int sp[kWarps];
   __shared__ float sv[kWarps];
