@@ -84,7 +84,11 @@ struct SpectralBins {
 #pragma unroll
       for (int l = 0; l < NL; ++l) {
         // a peak of 0 (intpolpeak ? ... : 0, nn:204) is staged as all zeros and adds nothing
-        const float sc = __fdividef(2.0f, pw[l].y);  // exp(-4 ln2 (d/w)^2) = 2^(-(2d/w)^2)
+        // exp(-4 ln2 (d/w)^2) = 2^(-(2d/w)^2); one Newton step takes the quotient's 2 ulp, which the exponent
+        // doubles, to half an ulp (not where w is 0 or out of range)
+        float sc = __fdividef(2.0f, pw[l].y);
+        const float rest = fmaf(-pw[l].y, sc, 2.0f);
+        if (fabsf(rest) < 1e-3f) sc = fmaf(0.5f * sc, rest, sc);
         sh.runs[l][d] = pw[l].x != 0.0f ? make_float4(pw[l].x * cnt, sc, -(vlos * shk[l]) * sc, 0.0f)
                                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
@@ -148,7 +152,8 @@ struct SpectralBins {
         for (int m = 0; m < NB; ++m) {
           const int il = wlo + m * 32 + lane;
           if (m < nw[l] && il < L) {
-            const float v = __double2float_rn(__dmul_rn(scale, (double)acc[l][m]));
+            // the sum with what its last additions dropped
+            const float v = __double2float_rn(__dmul_rn(scale, __dsub_rn((double)acc[l][m], (double)comp[l][m])));
             if (ATOMIC)
               atomicAdd(out + FOMO_IDX(ray * L + il, ncube, kSiteCube), v);
             else
