@@ -3077,7 +3077,8 @@ int march_bins_per_lane(int nlines, int L) {
 // passes add the deferred samples' emission with atomics.
 cudaError_t launch_march(const MarchArgs& a, const double3* ktab, int ktab_stride, int max_windows, int sm_count,
                          cudaStream_t s, int blocks_per_sm_hint, bool imaging, MarchTimer* timer) {
-  if (!a.deferred || a.deferred_cap <= 0 || !a.counter) return cudaErrorInvalidValue;
+  // (a radius of 0 would leave every sample to the lane walks)
+  if (!a.deferred || a.deferred_cap <= 0 || !a.counter || !(a.rscale > 0.0f)) return cudaErrorInvalidValue;
   const int kind = a.s2 ? kDeferredThomson : (imaging ? kDeferredImaging : kDeferredSpectral);
   auto mark = [&](int k) {
     if (timer) timer->mark(s, k);

@@ -179,6 +179,8 @@ extern "C" int fomo_render_noalloc(fomo_ctx* ctx, const fomo_request* req, float
   a.counter = counter;
   a.deferred = reinterpret_cast<DeferredRec*>(base + kOffDeferred);
   a.deferred_cap = kNoAllocDeferredCap;
+  a.rscale = search_radius(snap, 0.0f);
+  a.stats = ctx->march_stats;
   const int64_t chunk = kNoAllocDeferredCap / ((q.nz + 63) / 64);  // rays whose segments fit the queue
   for (int64_t b = 0; b < hoff[1] && e == cudaSuccess; b += chunk) {
     a.item_base = b;

@@ -847,6 +847,9 @@ bool bundle_view(const SnapRec& snap, const fomo_request& q, int tw, int th, boo
 // 40K points, 149 x 100 x 300 pixels 271 / 264 / 272 / 262 / 277 us; clustered: 8M-point rope, 1024^3
 // 23.9 / - / 22.2 / 21.4 / 20.9 ms (1.25: 21.6), its Thomson view - / - / 103.5 / 101.4 / 98.9 ms.
 constexpr float kRadiusUniform = 0.87f, kRadiusClustered = 1.1f;
+float search_radius(const SnapRec& snap, float wanted) {
+  return wanted > 0.0f ? wanted : (snap.uniform ? kRadiusUniform : kRadiusClustered);
+}
 
 // Plan a batch.  Requests are grouped into launches by (snapshot, method,
 // imaging); inside a launch, requests with the same view (angles, resolution,
@@ -958,7 +961,6 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     G.th = ctx->tile_h;
     G.bps = ctx->blocks_per_sm;
     G.rscale = ctx->rscale;
-    G.uniform = snap.uniform;
     if (G.tw <= 0 || G.th <= 0) {
       G.tw = 8;
       G.th = 4;
@@ -1219,7 +1221,7 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
     a.s2 = s2;
     a.totpol = G.totpol;
     a.stats = ctx->march_stats;
-    a.rscale = G.rscale > 0.0f ? G.rscale : (G.uniform ? kRadiusUniform : kRadiusClustered);
+    a.rscale = search_radius(snap, G.rscale);
     a.stop = scr->stop;
     if (e == cudaSuccess && scr->ev0 && ctx->time_march) e = record_timing(scr->ev0);
     MarchTimer* timer = (ctx->kernel_timing && !capturing) ? &ctx->timer : nullptr;

@@ -109,7 +109,6 @@ struct PlanGroup {
   int max_nw = 1;  // largest number of 32-bin lambda windows of a line
   int tw = 8, th = 4, bps = 0;
   float rscale = 0.0f;
-  bool uniform = false;  // the snapshot's points are close to uniform at the cell scale
   std::vector<const float2*> ew;       // payload per request (NN)
   const float2* totpol = nullptr;      // Thomson payload
   bool any_nn = false;
@@ -234,6 +233,8 @@ int issue_plan(fomo_ctx* ctx, const Plan& plan, ScratchSet* scr, cudaStream_t s,
 std::string workload_class(const PlanGroup& G, const SnapRec& snap);
 int order_streams(fomo_ctx* ctx, cudaStream_t s);
 SnapDev snap_dev(const SnapRec& r);
+// The search's gather radius in local point spacings: `wanted` where that is set (> 0), else the cloud's default.
+float search_radius(const SnapRec& snap, float wanted);
 float payload_wmax(fomo_ctx* ctx, int snap, int table, int imaging, double abund);
 void line_window(double lwa, int L, double lambda0, float vmax, float wmax, int* wstart, int* nw);
 void fill_view_host(const fomo_request& q, double lambda0, int tw, int th, ViewDesc* V);
