@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 
 namespace fomo {
@@ -82,11 +83,13 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// Kahan-compensated FP32 accumulation.
+// Kahan-compensated FP32 accumulation.  A sum that is infinite keeps no rest (it would be NaN, and the sum with the next
+// term too).
 __device__ __forceinline__ void kahan_add(float& sum, float& comp, float v) {
   const float y = __fsub_rn(v, comp);
   const float t = __fadd_rn(sum, y);
-  comp = __fsub_rn(__fsub_rn(t, sum), y);
+  const float rest = __fsub_rn(__fsub_rn(t, sum), y);
+  comp = fabsf(t) <= FLT_MAX ? rest : 0.0f;
   sum = t;
 }
 

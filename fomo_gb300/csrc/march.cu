@@ -1953,11 +1953,11 @@ __global__ void __launch_bounds__(kThreads, kMinCtasShade)
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
         const float so = __shfl_xor_sync(kFull, s, o), co = __shfl_xor_sync(kFull, c, o);
-        // s + so with its rounding error (two-sum); comp holds what a sum has too much
+        // s + so with its rounding error (two-sum; none of an infinite sum); comp holds what a sum has too much
         const float t = __fadd_rn(s, so), bb = __fsub_rn(t, s);
         const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(so, bb));
         s = t;
-        c = __fsub_rn(__fadd_rn(c, co), e);
+        c = __fsub_rn(__fadd_rn(c, co), fabsf(t) <= FLT_MAX ? e : 0.0f);
       }
       if (lane == 0)
         LD[l].out[FOMO_IDX(ray, (int64_t)V->nx * V->ny, kSiteCube)] = __double2float_rn(
