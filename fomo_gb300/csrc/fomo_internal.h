@@ -182,7 +182,8 @@ cudaError_t launch_bin_points(const float* x, const float* y, const float* z, in
                               int* cell_of, int* counts, cudaStream_t s);
 cudaError_t launch_block_bounds(const float4* pts, const int* cell_start, GridParams g, int bdx, int bdy, int bdz,
                                 float* blk, cudaStream_t s);
-cudaError_t launch_count_empty(const int* counts, int64_t ncells, unsigned long long* empty, cudaStream_t s);
+// out[0]: empty cells, out[1]: points of the fullest cell.
+cudaError_t launch_cell_stats(const int* counts, int64_t ncells, unsigned long long* out, cudaStream_t s);
 cudaError_t launch_exclusive_scan(const int* in, int* out, int64_t count, int* scratch, int64_t scratch_ints,
                                   cudaStream_t s);
 int64_t exclusive_scan_scratch_ints(int64_t count);

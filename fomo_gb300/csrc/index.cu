@@ -277,20 +277,34 @@ cudaError_t launch_block_bounds(const float4* pts, const int* cell_start, GridPa
   return cudaGetLastError();
 }
 
-// The number of cells whose count is 0 (added to *empty, zeroed by the caller).
-__global__ void count_empty_kernel(const int* __restrict__ counts, int64_t ncells, unsigned long long* empty) {
-  unsigned long long k = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncells; i += (int64_t)gridDim.x * blockDim.x)
-    k += counts[i] == 0 ? 1ull : 0ull;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) k += __shfl_xor_sync(0xffffffffu, k, o);
-  if ((threadIdx.x & 31) == 0 && k) atomicAdd(empty, k);
+// out[0]: the cells whose count is 0; out[1]: the largest count (both zeroed before).  Two atomics per block.
+__global__ void __launch_bounds__(256) cell_stats_kernel(const int* __restrict__ counts, int64_t ncells, unsigned long long* out) {
+  __shared__ unsigned int empty, fullest;
+  if (threadIdx.x == 0) empty = fullest = 0u;
+  __syncthreads();
+  unsigned int k = 0u, m = 0u;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < ncells; i += (int64_t)gridDim.x * blockDim.x) {
+    const unsigned int c = (unsigned int)counts[i];
+    k += c == 0u;
+    m = max(m, c);
+  }
+  k = __reduce_add_sync(0xffffffffu, k);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&empty, k);
+    atomicMax(&fullest, m);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicAdd(out, (unsigned long long)empty);
+    atomicMax(out + 1, (unsigned long long)fullest);
+  }
 }
 
-cudaError_t launch_count_empty(const int* counts, int64_t ncells, unsigned long long* empty, cudaStream_t s) {
-  cudaError_t e = cudaMemsetAsync(empty, 0, sizeof(unsigned long long), s);
+cudaError_t launch_cell_stats(const int* counts, int64_t ncells, unsigned long long* out, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(out, 0, 2 * sizeof(unsigned long long), s);
   if (e != cudaSuccess) return e;
-  count_empty_kernel<<<grid_blocks(ncells, 256), 256, 0, s>>>(counts, ncells, empty);
+  cell_stats_kernel<<<std::min(grid_blocks(ncells, 256), 152 * 4), 256, 0, s>>>(counts, ncells, out);
   return cudaGetLastError();
 }
 

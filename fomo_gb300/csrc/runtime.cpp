@@ -421,6 +421,7 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   // skips the choice.
   double ppc = ctx->cell_occupancy;
   bool uniform = false;
+  int64_t fullest = n;
   if (!ctx->occupancy_set && n >= 1024) {
     const GridParams g2 = choose_grid(mn, mx, n, 2.0);
     const int64_t nc2 = (int64_t)g2.dx * g2.dy * g2.dz;
@@ -431,19 +432,20 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
       dev_free(ctx, bits);
       return rc;
     }
-    unsigned long long hempty = 0;
-    unsigned long long* dempty = reinterpret_cast<unsigned long long*>(bits);
+    unsigned long long hstats[2] = {0, 0};  // empty cells, points of the fullest
+    unsigned long long* dstats = reinterpret_cast<unsigned long long*>(bits);
     e = cudaMemsetAsync(t2 + n, 0, sizeof(int) * (size_t)nc2, s);
     if (e == cudaSuccess) e = launch_bin_points(a[0], a[1], a[2], n, g2, t2, t2 + n, s);
-    if (e == cudaSuccess) e = launch_count_empty(t2 + n, nc2, dempty, s);
-    if (e == cudaSuccess) e = read_back(ctx, &hempty, dempty, sizeof(hempty), s);
+    if (e == cudaSuccess) e = launch_cell_stats(t2 + n, nc2, dstats, s);
+    if (e == cudaSuccess) e = read_back(ctx, hstats, dstats, sizeof(hstats), s);
     dev_free(ctx, t2, e == cudaSuccess);
     if (e != cudaSuccess) {
       dev_free(ctx, stage);
       dev_free(ctx, bits);
       return cuda_err(ctx, e, "snapshot cell statistics");
     }
-    uniform = (double)hempty < kUniformEmpty * (double)nc2;
+    uniform = (double)hstats[0] < kUniformEmpty * (double)nc2;
+    fullest = (int64_t)hstats[1];
     ppc = uniform ? 1.0 : 2.0;
   }
   float spacing = 0.0f;
@@ -470,6 +472,7 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   R.g = g;
   R.spacing = spacing;
   R.uniform = uniform;
+  R.fullest = fullest;
   const int bdx = (g.dx + kBlockCells - 1) / kBlockCells, bdy = (g.dy + kBlockCells - 1) / kBlockCells,
             bdz = (g.dz + kBlockCells - 1) / kBlockCells;
   const int64_t nblk = (int64_t)bdx * bdy * bdz;
@@ -519,6 +522,12 @@ int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec
   *out = R;
   return FOMO_OK;
 }
+
+// Points of a cloud's fullest cell (at two points per cell) up to which every lane walk over a narrow box is short:
+// half the 48 points in a row of cells at which a budgeted walk hands its sample to a warp.  Regular and jittered grids hold
+// up to 12; the share of empty cells says nothing of a few dense knots.  64^3 points plus 10 % in eight knots (cells of 2,700
+// points), 256^2 x 256 and 512^2 x 512: without the queue 4,900 and 7,900 us, with it 1,100 and 2,700.
+constexpr int64_t kFullestShort = 24;
 
 SnapDev snap_dev(const SnapRec& r) {
   SnapDev s;
@@ -1009,12 +1018,12 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
     G.deferred_cap = deferred_capacity(items, G.maxnz);
     G.o_def = L.take(sizeof(DeferredRec) * (size_t)G.deferred_cap);
     // Boxes narrower than kFarBox cells in every view (md = pitch / 0.3, nn:138): no half record
-    // can be listed for the far pass.  In a cloud close to uniform a lane's walk over such a box
-    // is short as well, and needs no queue of hard samples.  Either pass is a launch of 3 to 5 us
-    // that finds its queue empty.
+    // can be listed for the far pass.  In a cloud close to uniform without dense cells a lane's walk
+    // over such a box is short as well, and needs no queue of hard samples.  Either pass is a launch of
+    // 3 to 5 us that finds its queue empty.
     bool wide = G.method == FOMO_METHOD_THOMSON;
     for (auto& v : G.vreqs) wide = wide || view_pitch(snap, reqs[v[0]]) / 0.3 * 1.0001 >= kFarBox * snap.g.h;
-    G.hard_cap = wide || !snap.uniform ? hard_capacity(items, G.maxnz) : 0;
+    G.hard_cap = wide || !snap.uniform || snap.fullest > kFullestShort ? hard_capacity(items, G.maxnz) : 0;
     G.o_hard = L.take(sizeof(uint2) * (size_t)G.hard_cap);
     // the searches and the emission run as separate passes through a
     // neighbour buffer (each pass at its own occupancy; the emission pass runs

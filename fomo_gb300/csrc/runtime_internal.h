@@ -46,6 +46,7 @@ struct SnapRec {
   GridParams g{};
   float spacing = 0.0f;   // mean point spacing: (volume / points)^(1/3) over the axes with an extent
   bool uniform = false;   // few empty cells: close to uniform at the cell scale
+  int64_t fullest = 0;    // points of the fullest cell at two points per cell (n where that is not looked at)
   void* block = nullptr;  // one allocation for everything below
   size_t bytes = 0;
   float4* pts = nullptr;
