@@ -2140,19 +2140,23 @@ __device__ __forceinline__ bool box_cells(const GridParams& g, const BoxQ& q, in
   return true;
 }
 
-// Rows + points one lane may scan for one sample before a warp takes it.  Deferred / hard pass at 192, 128, 96, 64: 24 views
-// of 64^2 to 700^2 pixels one after the other 7.7 / 2.35, 7.2 / 2.40, 7.0 / 2.44, 6.5 / 2.68 ms (the longest walk is the deferred pass's
-// time there); with range bounds of 32 and 24 points in place of kLaneDense no better.
-constexpr int kLaneBudget = 64;
+// Rows + points one lane may scan for one sample before a warp takes it.  With warps waiting for samples the deferred pass
+// lasts as long as its longest walk, and a short budget is the faster: deferred / hard pass at 192, 128, 96, 64: 24 views of 64^2
+// to 700^2 pixels one after the other 7.7 / 2.35, 7.2 / 2.40, 7.0 / 2.44, 6.5 / 2.68 ms; range bounds of 32 and 24 points in
+// place of kLaneDense were no better.  Once kHardShort samples are queued (20 for each warp of the hard pass) a warp per
+// sample is the dearer way: a cloud of 64^3 points and eight knots, 101 x 102 x 300, queues 281,000 samples at 64 and 1,700
+// at 192, the render takes 1380 and 810 us, and 1150 with both budgets.  A shorter queue gives 1075 (65,536) and 1020 us (32,768)
+// there, but views of 48^2, whose whole queue is of that length, then wait for late long walks (892 -> 945, 960 -> 1080 us).
+constexpr int kLaneBudget = 64, kLaneBudgetLong = 192;
+constexpr unsigned long long kHardShort = 98304;
 
 // Nearest point strictly inside box q, searched by this lane alone: sorted
 // position and original index, or -1 when the box holds no point.  With
-// BUDGET, false when the search ran out of kLaneBudget (dense cells, or a
+// BUDGET, false when the search ran out of its budget (dense cells, or a
 // wide box far from the points): a whole warp then searches the sample
 // (warp_search, march_hard).
 template <bool BUDGET>
-__device__ __forceinline__ bool lane_search(const SnapDev& S, const BoxQ& q, int& pos, int& orig) {
-  int budget = kLaneBudget;
+__device__ __forceinline__ bool lane_search(const SnapDev& S, const BoxQ& q, int& pos, int& orig, int budget = 0) {
   pos = -1;
   orig = -1;
   int b0[3], b1[3], c[3];
@@ -2823,7 +2827,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasFar) march_far(MarchArgs a, 
 template <bool BUDGET, bool POS>
 __device__ __forceinline__ void deferred_search(const MarchArgs& a, int kind, int nsamp, int start, int incl,
                                                 int excl, const DeferredRec& rec, const RayCtx& mine, int stride,
-                                                int* sp, float* sv) {
+                                                int* sp, float* sv, int& budget) {
   const int lane = threadIdx.x & 31;
   for (int t0 = 0; t0 < nsamp; t0 += 32) {
     const int t = t0 + lane;
@@ -2836,13 +2840,14 @@ __device__ __forceinline__ void deferred_search(const MarchArgs& a, int kind, in
     int k = 0, p = -1, o = -1;
     if (t < nsamp) {
       k = (int)oy + nth_set_bit(oz, ow, start + t - oe);
-      hard = !lane_search<BUDGET>(a.snap, exact_box(r, k), p, o);
+      hard = !lane_search<BUDGET>(a.snap, exact_box(r, k), p, o, budget);
     }
     if (BUDGET) {
       const unsigned hm = __ballot_sync(kFull, hard);
       unsigned long long hb = 0;
       if (hm && lane == 0) hb = atomicAdd(a.counter + kCtrHard, (unsigned long long)__popc(hm));
       hb = __shfl_sync(kFull, hb, 0);
+      if (hb >= kHardShort) budget = kLaneBudgetLong;
       if (hard) {
         const int64_t slot = (int64_t)hb + __popc(hm & ((1u << lane) - 1u));
         if (slot < a.hard_cap) {
@@ -2891,6 +2896,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasDeferred) march_deferred(Mar
   const int grab = (int)max((int64_t)1, min((int64_t)32, nrec / nwarps));
   // a short queue (a small render: latency matters) takes the budgeted search
   const bool budgeted = a.hard_cap > 0 && nrec < 256 * nwarps;
+  int budget = kLaneBudget;  // of this warp's walks, until it sees that the hard queue is long
   for (;;) {
     unsigned long long base = 0;
     if (lane == 0) base = atomicAdd(a.counter + kCtrDeferredHead, (unsigned long long)grab);
@@ -2915,9 +2921,9 @@ __global__ void __launch_bounds__(kThreads, kMinCtasDeferred) march_deferred(Mar
       const int nsamp = __shfl_sync(kFull, incl, r1 - 1) - start;
       // 1. one sample per lane: its record, ray and box, then its own search
       if (budgeted)
-        deferred_search<true, POS>(a, kind, nsamp, start, incl, excl, rec, mine, ktab_stride, spos[w], svlos[w]);
+        deferred_search<true, POS>(a, kind, nsamp, start, incl, excl, rec, mine, ktab_stride, spos[w], svlos[w], budget);
       else
-        deferred_search<false, POS>(a, kind, nsamp, start, incl, excl, rec, mine, ktab_stride, spos[w], svlos[w]);
+        deferred_search<false, POS>(a, kind, nsamp, start, incl, excl, rec, mine, ktab_stride, spos[w], svlos[w], budget);
       if (!POS) {
         __syncwarp();
         // 2. their emission, record by record
