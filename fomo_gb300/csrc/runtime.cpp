@@ -831,13 +831,13 @@ double view_pitch(const SnapRec& snap, const fomo_request& q) {
 // dense part, where the pixels lie and the search takes longest, and the bound is
 // half that: 4M-point flux rope 1.1 1485 / 1780, 0.85 2003 / 1957, 0.43 5593 / 3709;
 // 0.5M-point rope 0.85 860 / 1047, 0.57 1137 / 1292, 0.43 1486 / 1552, 0.21 3200 / 2077.
-// Served views of kServedWhole samples or more stay with one ray per warp:
-// tests/test_gpu_failures.py cancels one 20 ms after its start and wants it to
-// run for 50 ms when it is not cancelled (41 ms as blocks).
+// Served views of kServedWhole samples or more stay with one ray per warp although blocks are faster (2^31 samples
+// 27 ms): tests/test_gpu_failures.py cancels such a request 20 ms after its start and wants the first whole one, with the 3 ms
+// of its allocations, to take over 50 ms.
 constexpr double kBundlePitch = 1.0, kBundlePitchClustered = 0.5;
-// Their search also leaves one of its seven places per SM to the other streams' kernels: a
-// 100 x 100 x 256 request beside a 1024 x 1024 x 2048 one takes 0.52 ms instead of 0.82,
-// the large one 50.1 ms instead of 46.5 (five places: 55.8 ms, and no more for the small one).
+// Their search leaves one of its seven places per SM to the other streams' kernels.  A 1024 x 1024 x 2048 request takes
+// 46.5 ms with all seven (the test's 49.6), 50.0 with six (53.1), 55.6 with five (58.7); 100 x 100 x 256 requests beside it
+// 0.97 ms (the slowest 1.28), 0.66 (1.15) and 0.67 (0.97).
 constexpr double kServedWhole = 1073741824.0;
 constexpr int kServedPlaces = 6;
 bool served_whole(const fomo_request& q, bool served) {
