@@ -28,7 +28,7 @@ std::string plan_key(const Plan& p, const ScratchSet& scr) {
   for (const PlanGroup& G : p.groups) {
     k << "|" << G.snapshot << "," << G.method << "," << G.imaging << "," << G.nv << "," << G.nl << "," << G.maxL
       << "," << G.maxnz << "," << G.maxnx << "," << G.maxny << "," << G.total_items << "," << G.tw << "," << G.th
-      << "," << G.bps << "," << G.rscale << "," << G.any_nn << "," << G.item_off[G.bundle_view] << "," << (const void*)G.totpol << "," << G.max_nw << "," << G.hard_cap << "," << G.o_far;
+      << "," << G.bps << "," << G.rscale << "," << G.any_nn << "," << G.item_off[G.bundle_view] << "," << (const void*)G.totpol << "," << G.max_nw << "," << G.hard_cap << "," << G.o_far << "," << G.by_pixel;
     // launches that hold a view's size or an output
     if (G.method == FOMO_METHOD_PROJECTION)
       for (int64_t n : G.npix) k << "," << n;

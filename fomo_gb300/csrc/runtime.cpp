@@ -717,6 +717,11 @@ size_t cube_elems(const fomo_request& q) {
   return (size_t)q.nx * q.ny * (q.method == FOMO_METHOD_THOMSON ? 1 : q.nlambda);
 }
 
+size_t projection_list_bytes(int64_t n, int64_t npix) {
+  return sizeof(int) * (2 * (size_t)(npix + 1) + (size_t)exclusive_scan_scratch_ints(npix + 1) + (size_t)n) +
+         sizeof(int2) * ((size_t)n + (size_t)projection_pieces(n)) + 6 * 256;
+}
+
 void fill_view_host(const fomo_request& q, double lambda0, int tw, int th, ViewDesc* V) {
   std::memset(V, 0, sizeof(*V));
   V->cb = std::cos(q.b);
@@ -1039,24 +1044,39 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
       if (wide) G.o_far = L.take(sizeof(int32_t) * (size_t)G.deferred_cap);
       G.o_ktf = L.take(sizeof(float2) * 3 * (size_t)G.nv * G.maxnz);
     }
-    if (G.method == FOMO_METHOD_PROJECTION) {
-      // (the windows are known after the descriptors are filled: room for the widest lines)
-      G.by_pixel = projection_by_pixel(snap.n, G.nl, G.imaging ? 1 : (G.maxL + 31) / 32, G.imaging != 0);
-      if (G.by_pixel) {
-        const size_t npix = (size_t)G.maxnpix + 1;
-        G.o_pcount = L.take(sizeof(int) * npix);
-        G.o_pfirst = L.take(sizeof(int) * npix);
-        G.o_pscan = L.take(sizeof(int) * (size_t)exclusive_scan_scratch_ints((int64_t)npix));
-        G.o_pat = L.take(sizeof(int2) * (size_t)snap.n);
-        G.o_plist = L.take(sizeof(int) * (size_t)snap.n);
-        G.o_ppieces = L.take(sizeof(int2) * (size_t)projection_pieces(snap.n));
-      }
-    }
     G.o_s2 = G.method == FOMO_METHOD_THOMSON ? L.take(sizeof(float) * (size_t)G.nv * snap.n) : 0;
   }
-  plan->dev_bytes = L.off;
-  int rc = scr->arena.reserve(ctx, plan->dev_bytes);
+  // Projections that list their points by pixel: the lists come last, so that where the budget, the device or what a
+  // server admitted does not hold them these projections go by the direct kernel, which needs none.
+  const size_t without = L.off;
+  size_t room = scr->list_room;
+  for (PlanGroup& G : plan->groups) {
+    const int64_t n = ctx->snaps[G.snapshot].n;
+    const size_t npix = (size_t)G.maxnpix + 1, bytes = projection_list_bytes(n, G.maxnpix);
+    // (the windows are known after the descriptors are filled: room for the widest lines)
+    G.by_pixel = G.method == FOMO_METHOD_PROJECTION && bytes <= room &&
+                 projection_by_pixel(n, G.nl, G.imaging ? 1 : (G.maxL + 31) / 32, G.imaging != 0);
+    if (!G.by_pixel) continue;
+    room -= bytes;
+    G.o_pcount = L.take(sizeof(int) * npix);
+    G.o_pfirst = L.take(sizeof(int) * npix);
+    G.o_pscan = L.take(sizeof(int) * (size_t)exclusive_scan_scratch_ints((int64_t)npix));
+    G.o_pat = L.take(sizeof(int2) * (size_t)n);
+    G.o_plist = L.take(sizeof(int) * (size_t)n);
+    G.o_ppieces = L.take(sizeof(int2) * (size_t)projection_pieces(n));
+  }
+  auto drop_lists = [&] {
+    for (PlanGroup& G : plan->groups) G.by_pixel = false;
+    L.off = without;
+  };
+  if (L.off > scr->arena.cap && ctx->used - scr->arena.cap + L.off > ctx->budget) drop_lists();
+  int rc = scr->arena.reserve(ctx, L.off);
+  if (rc == FOMO_ENOMEM && L.off > without) {
+    drop_lists();
+    rc = scr->arena.reserve(ctx, L.off);
+  }
   if (rc) return rc;
+  plan->dev_bytes = L.off;
   rc = scr->staging.reserve(ctx, plan->host_bytes);
   if (rc) return rc;
   if (scr->staging.copy_done) cudaEventSynchronize(scr->staging.copy_done);  // previous upload has run

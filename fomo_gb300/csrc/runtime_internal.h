@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <nvtx3/nvToolsExt.h>
 
+#include <stdint.h>
+
 #include <functional>
 #include <map>
 #include <string>
@@ -82,6 +84,7 @@ struct ScratchSet {
   Arena arena;
   Staging staging;
   unsigned* stop = nullptr;  // a server slot's stop word (device), null for the context's own batches
+  size_t list_room = SIZE_MAX;  // bytes that projections may take to list their points by pixel (a server: those admitted)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaError_t init() {
     cudaError_t e = cudaEventCreate(&ev0);
@@ -218,6 +221,8 @@ void dev_free(fomo_ctx* ctx, void* p, bool idle = false);
 void release_free_blocks(fomo_ctx* ctx);  // cudaFree of the blocks dev_free kept
 int validate(fomo_ctx* ctx, const fomo_request& q);
 size_t cube_elems(const fomo_request& q);
+// Scratch of a projection of n points that lists them by pixel.
+size_t projection_list_bytes(int64_t n, int64_t npix);
 // Called by issue_plan once the work of views [v0, v1) of launch G is on the
 // stream: their cubes are complete when the stream reaches that point.  With
 // it, a launch marches in view ranges: ranges of about `range_cost` LOS

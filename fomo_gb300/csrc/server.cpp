@@ -54,6 +54,7 @@ struct Ticket {
   float* out_host = nullptr;
   size_t out_bytes = 0;
   size_t cost = 0;  // admission bytes
+  size_t list = 0;  // of these, for listing a projection's points by pixel
   TState state = TState::kQueued;
   bool cancelled = false;
   int status = FOMO_OK;
@@ -130,6 +131,18 @@ size_t request_cost(const fomo_request& q) {
          (q.method != FOMO_METHOD_PROJECTION  // neighbour buffer and far-pass list
               ? rays * (size_t)q.nz * sizeof(int32_t) + rays * (size_t)((q.nz + 63) / 64) * sizeof(int32_t)
               : 0);
+}
+
+// Bytes a projection takes beyond that where it lists its points by pixel (requests of one view share them; up to four
+// lines of a view may come together).  A request whose lists do not fit the budget goes without (plan_batch).
+size_t list_cost(fomo_server* S, const fomo_request& q) {
+  const auto it = S->ctx->snaps.find(q.snapshot);
+  if (q.method != FOMO_METHOD_PROJECTION || it == S->ctx->snaps.end()) return 0;
+  const int64_t n = it->second.n;
+  const int windows = (q.nlambda + 31) / 32;
+  bool listed = false;
+  for (int nl = 1; nl <= 4; ++nl) listed = listed || projection_by_pixel(n, nl, windows, q.nlambda <= 1);
+  return listed ? projection_list_bytes(n, (int64_t)q.nx * q.ny) : 0;
 }
 
 // Requests `ids` of slot sl are complete (their cubes are in pinned staging);
@@ -269,6 +282,7 @@ void scheduler(fomo_server* S) {
       std::vector<fomo_request> reqs;
       std::vector<size_t> out_bytes;
       const double t = now_s() - S->t0;
+      free_slot->scr.list_room = 0;
       while (!S->queue.empty()) {
         uint64_t id = S->queue.front();
         Ticket& T = S->tickets[id];
@@ -288,6 +302,7 @@ void scheduler(fomo_server* S) {
         S->inflight_bytes += T.cost;
         S->inflight += 1;
         free_slot->cost += T.cost;
+        free_slot->scr.list_room += T.list;
         ids.push_back(id);
         reqs.push_back(T.req);
         out_bytes.push_back(T.out_bytes);
@@ -387,6 +402,9 @@ int fomo_server_submit(fomo_server* S, const fomo_request* req, float* out_host,
     S->err = "server is stopping";
     return FOMO_ECANCELLED;
   }
+  T.list = list_cost(S, *req);
+  if (T.cost + T.list > S->budget) T.list = 0;
+  T.cost += T.list;
   T.t_submit = now_s() - S->t0;
   const uint64_t id = S->next_ticket++;
   S->tickets[id] = T;
