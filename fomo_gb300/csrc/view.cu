@@ -289,20 +289,21 @@ __device__ __forceinline__ float2 fp32_pair(double v) {
   return make_float2(hi, __double2float_rn(__dsub_rn(v, (double)hi)));
 }
 
-// grid: (views, 1 + chunks of kTabChunk table entries).  Block (v, 0) fills the
+// grid: (1 + chunks of kTabChunk table entries, views): an image side may have more chunks than
+// the 65,535 of the grid's y axis.  Block (0, v) fills the
 // view's scalars, independent chains of FP64 divisions on lanes of their own
 // (on one thread, with the tables after them in the same block: 10 us per launch,
 // an FP64 division taking about 0.7); the others fill the tables of ray x, ray y
 // and LOS positions, one entry per thread, from the extents.
 constexpr int kTabChunk = 128;
 __global__ void __launch_bounds__(kTabChunk) view_finalize_kernel(ViewDesc* views, double3* ktab, float2* ktf, int ktab_stride) {
-  ViewDesc* V = views + blockIdx.x;
+  ViewDesc* V = views + blockIdx.y;
   const double minx = ord2d(V->ext_bits[0]), maxx = ord2d(V->ext_bits[1]);
   const double miny = ord2d(V->ext_bits[2]), maxy = ord2d(V->ext_bits[3]);
   const double minz = ord2d(V->ext_bits[4]), maxz = ord2d(V->ext_bits[5]);
   const double dxr = __dsub_rn(maxx, minx), dyr = __dsub_rn(maxy, miny);
   const int nx = V->nx, ny = V->ny, nz = V->nz;
-  if (blockIdx.y == 0) {
+  if (blockIdx.x == 0) {
     __shared__ double s_px, s_py;
     if (threadIdx.x == 0) {
       V->minx = minx;
@@ -352,14 +353,14 @@ __global__ void __launch_bounds__(kTabChunk) view_finalize_kernel(ViewDesc* view
     }
     return;
   }
-  int i = (blockIdx.y - 1) * kTabChunk + threadIdx.x;
+  int i = (blockIdx.x - 1) * kTabChunk + threadIdx.x;
   if (i < nz) {
     double dz = __dsub_rn(maxz, minz);
     if (nz != 1) dz = __ddiv_rn(dz, (double)(nz - 1));
     const double z = __dadd_rn(__dmul_rn((double)i, dz), minz);  // nn:162
     const double zsb = __dmul_rn(z, V->sb);
     const double3 t = make_double3(__dmul_rn(zsb, V->cl), __dmul_rn(zsb, V->sl), __dmul_rn(z, V->cb));
-    const int64_t k = (int64_t)blockIdx.x * ktab_stride + FOMO_IDX(i, ktab_stride, kSiteKtab);
+    const int64_t k = (int64_t)blockIdx.y * ktab_stride + FOMO_IDX(i, ktab_stride, kSiteKtab);
     ktab[k] = t;
     if (ktf) {
       float2* f = ktf + 3 * k;
@@ -407,7 +408,7 @@ cudaError_t launch_view_extents(SnapDev snap, ViewDesc* views, int nviews, float
 cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, float2* ktf, int ktab_stride,
                                  int max_entries, cudaStream_t s) {
   const unsigned chunks = (unsigned)((max_entries + kTabChunk - 1) / kTabChunk);
-  view_finalize_kernel<<<dim3((unsigned)nviews, 1 + chunks), kTabChunk, 0, s>>>(views, ktab, ktf, ktab_stride);
+  view_finalize_kernel<<<dim3(1 + chunks, (unsigned)nviews), kTabChunk, 0, s>>>(views, ktab, ktf, ktab_stride);
   return cudaGetLastError();
 }
 
