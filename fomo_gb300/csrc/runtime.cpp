@@ -5,6 +5,7 @@
 // descriptors and outputs), orchestrates the kernels of index.cu, emission.cu,
 // view.cu and march.cu on one CUDA stream, and maps every failure to a
 // negative status with a message (the reference exits instead).
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -24,6 +25,7 @@
 #include <vector>
 
 #include "../../include/fomo_gpu.h"
+#include "array_in_place.h"
 #include "fomo_internal.h"
 #include "runtime_internal.h"
 
@@ -349,20 +351,37 @@ cudaError_t read_back(fomo_ctx* ctx, void* dst, const void* src, size_t bytes, c
   return e;
 }
 
+// array_in_place, with the allocation as the driver knows it (no such answer: false).
+bool readable_in_place(const void* p, size_t bytes) {
+  using Query = CUresult(CUDAAPI*)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    const cudaError_t e = cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found);
+    return e == cudaSuccess && found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(f) : nullptr;
+  }();
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* to[2] = {&base, &size};
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  return query && query(2, what, to, (CUdeviceptr)at) == CUDA_SUCCESS && array_in_place(at, bytes, (uintptr_t)base, size);
+}
+
 constexpr double kUniformEmpty = 0.10;  // empty-cell share below which a cloud counts as uniform
 
 int build_snapshot(fomo_ctx* ctx, int64_t n, const float* const host[8], SnapRec* out) {
   NvtxRange range("fomo: snapshot upload and index");
   cudaStream_t s = ctx->stream;
-  // staging for the host arrays (z may be absent -> zeros, as nn:82 for 2-D data); arrays in this
-  // device's memory are read where they are
+  // staging for the host arrays (z may be absent -> zeros, as nn:82 for 2-D data); arrays whole in this
+  // device's memory are read where they are, others (misaligned, or in several mappings) copied
   const float* a[8];
   int nstage = 0;
   for (int k = 0; k < 8; ++k) {
     a[k] = nullptr;
     cudaPointerAttributes at;
     if (host[k] && cudaPointerGetAttributes(&at, host[k]) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
-        at.device == ctx->device)
+        at.device == ctx->device && readable_in_place(host[k], sizeof(float) * (size_t)n))
       a[k] = host[k];
     else
       ++nstage;
