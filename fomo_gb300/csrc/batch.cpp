@@ -16,6 +16,7 @@
 
 #include "../../include/fomo_gpu.h"
 #include "runtime_internal.h"
+#include "tune_candidates.h"
 
 using namespace fomo;
 
@@ -104,7 +105,7 @@ int fomo_render_batch_graph(fomo_ctx* ctx, const fomo_request* reqs, int nreq, f
 // in the first pass, at more candidates per segment; a narrower one leaves more
 // to the deferred pass).  The segment length is fixed at 64 LOS samples (two
 // per lane) by the deferred-record format.  Cache file lines:
-// "<class> tile_w tile_h blocks_per_sm rscale ms".
+// "<class> tile_w tile_h blocks_per_sm rscale ms" (rscale 0: the default).
 int fomo_autotune(fomo_ctx* ctx, const fomo_request* reqs, int nreq, const char* cache_path) {
   if (!ctx || !reqs || nreq <= 0) return FOMO_EINVAL;
   NvtxRange range("fomo: autotune");
@@ -148,20 +149,21 @@ int fomo_autotune(fomo_ctx* ctx, const fomo_request* reqs, int nreq, const char*
   }
   const int saved_w = ctx->tile_w, saved_h = ctx->tile_h, saved_b = ctx->blocks_per_sm;
   const float saved_r = ctx->rscale;
-  // {tile_w, tile_h, CTA cap of the search, gather radius x 10}: tiles at the
-  // default search, then the search's occupancy and radius at the default tile
-  const int cands[][4] = {{8, 4, 0, 9},  {16, 2, 0, 9}, {4, 8, 0, 9},  {32, 1, 0, 9},  {8, 8, 0, 9},
-                          {8, 4, 6, 9},  {8, 4, 5, 9},  {8, 4, 0, 8},  {8, 4, 0, 10}, {8, 4, 0, 11}};
+  int blocks = 0, views = 0;  // views searched as blocks of rays, of all
+  for (const PlanGroup& G : probe.groups) {
+    blocks += G.nv - G.bundle_view;
+    views += G.nv;
+  }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   float best = 1e30f;
   TuneChoice bestc;
-  for (auto& c : cands) {
-    ctx->tile_w = c[0];
-    ctx->tile_h = c[1];
-    ctx->blocks_per_sm = c[2];
-    ctx->rscale = 0.1f * (float)c[3];
+  for (const TuneCandidate& c : tune_candidates(2 * blocks >= views ? kBundleCtas : kSearchCtas)) {
+    ctx->tile_w = c.tile_w;
+    ctx->tile_h = c.tile_h;
+    ctx->blocks_per_sm = c.cap;
+    ctx->rscale = c.radius;
     rc = enqueue_batch(ctx, reqs, nreq, d.data(), nullptr, ctx->stream, nullptr, nullptr);  // warm-up
     if (rc) break;
     cudaEventRecord(e0, ctx->stream);
@@ -177,7 +179,7 @@ int fomo_autotune(fomo_ctx* ctx, const fomo_request* reqs, int nreq, const char*
     cudaEventElapsedTime(&ms, e0, e1);
     if (ms < best) {
       best = ms;
-      bestc = TuneChoice{c[0], c[1], c[2], 0.1f * (float)c[3]};
+      bestc = TuneChoice{c.tile_w, c.tile_h, c.cap, c.radius};
     }
   }
   cudaEventDestroy(e0);

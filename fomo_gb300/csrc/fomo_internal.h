@@ -94,6 +94,9 @@ enum MarchCounter {
   kCtrCount
 };
 
+// CTAs per SM that the searches of single rays and of blocks of rays are built for.
+constexpr int kSearchCtas = 7, kBundleCtas = 5;
+
 // Box half-width, in cells, from which the far pass takes a view's samples (narrower: lane walks).
 constexpr float kFarBox = 4.0f;
 

@@ -87,8 +87,8 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kUnitsPerWarp = 8;
 constexpr int kMinCtasHard = 8;     // whole-warp walks: 32 warps at 64 registers (96^2 view of the 0.5M-point rope 101, 90, 85 us at 4, 6, 8 CTAs)
 constexpr int kMinCtas = 4;  // resident CTAs per SM: 16 warps of latency hiding at <= 128 registers
-constexpr int kMinCtasSearch = 7;   // the search-only pass: 28 warps at <= 72 registers (31 KB shared per CTA)
-constexpr int kMinCtasBundle = 5;   // the search over blocks of rays: 20 warps at <= 102 registers (at 64 views x 4 lines: 37.1, 35.4, 38.4, 37.7 ms at 4 to 7 CTAs)
+constexpr int kMinCtasSearch = kSearchCtas;   // the search-only pass: 28 warps at <= 72 registers (31 KB shared per CTA)
+constexpr int kMinCtasBundle = kBundleCtas;   // the search over blocks of rays: 20 warps at <= 102 registers (at 64 views x 4 lines: 37.1, 35.4, 38.4, 37.7 ms at 4 to 7 CTAs)
 constexpr int kMinCtasShade = 8;   // the emission-only pass: 32 warps at <= 64 registers
 constexpr int kMinCtasImaging = 5; // imaging / Thomson first pass: 20 warps at <= 102 registers
 constexpr int kMinCtasDeferred = 8; // one-lane ring walks wait on dependent loads: 32 warps (64 registers, some spill)
