@@ -22,10 +22,10 @@ using namespace fomo;
 
 namespace {
 
-std::string plan_key(const Plan& p, const ScratchSet& scr) {
+std::string plan_key(const Plan& p, const ScratchSet& scr, const void* counters) {
   std::ostringstream k;
   k << (const void*)scr.arena.base << "/" << (const void*)scr.staging.base << "/" << p.host_bytes << "/"
-    << p.dev_bytes;
+    << p.dev_bytes << "/" << counters;
   for (const PlanGroup& G : p.groups) {
     k << "|" << G.snapshot << "," << G.method << "," << G.imaging << "," << G.nv << "," << G.nl << "," << G.maxL
       << "," << G.maxnz << "," << G.maxnx << "," << G.maxny << "," << G.total_items << "," << G.tw << "," << G.th
@@ -65,7 +65,7 @@ int fomo_render_batch_graph(fomo_ctx* ctx, const fomo_request* reqs, int nreq, f
   if (rc) return rc;
   rc = order_after_ctx_stream(ctx, s);
   if (rc) return rc;
-  const std::string key = plan_key(plan, ctx->scratch);
+  const std::string key = plan_key(plan, ctx->scratch, ctx->march_stats);
   auto it = ctx->graphs.find(key);
   if (it == ctx->graphs.end()) {
     cudaGraph_t g = nullptr;
