@@ -1064,7 +1064,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasSearch) march_search(MarchAr
 //    of 32, 16 or 8 samples; where that does not do (points much denser than
 //    pixels), its rays go to march_split one by one.
 // ---------------------------------------------------------------------------
-constexpr int kBunCap = 208;  // candidates per part (sized so that 7 CTAs fit an SM)
+constexpr int kBunCap = 208;  // candidates per part: 30.5 KB of lists per CTA, 153 KB with kMinCtasBundle CTAs per SM
 
 struct __align__(16) BundleSmem {
   // [0, kBunCap): gathered candidates (x, y, z, sorted position); [kBunCap, 2 kBunCap):

@@ -13,8 +13,8 @@
 // __device__ array of fixed size, so a call never allocates.  The descriptors
 // reach the array as the parameter of a small kernel, not through a host
 // copy.  The queue's fixed capacity (65,536 segment records) makes a large
-// render march its rays in chunks; each chunk costs a counter clear and four
-// launches (first pass, split, deferred and hard passes), so a render at the
+// render march its rays in chunks; each chunk costs a counter clear and three
+// launches (first pass, split and deferred passes), so a render at the
 // limits (4096 x 4096 rays at nz = 4096: chunks of 1,024 rays) issues about
 // 16,000 chunks.
 //
@@ -24,7 +24,7 @@
 // device (that first call should therefore come before any stream capture).
 // Every call on a device shares the same array and the array keeps the last
 // call's contents: the work counters are cleared by each chunk, the per-view
-// extents are initialised by a kernel of each call, everything else is fully
+// extents start from the descriptors of each call, everything else is fully
 // rewritten.  Calls that overlap on the GPU (e.g. on two streams) race on the
 // array; serialise them.
 //

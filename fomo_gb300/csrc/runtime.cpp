@@ -1193,7 +1193,7 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
 // cost, one range per 64 MB of cubes, 8 at most.
 static std::vector<int> view_ranges(const PlanGroup& G, bool split, double range_cost) {
   if (split && range_cost > 0.0) {
-    // ranges of about range_cost each (views in plan order: smaller images first)
+    // ranges of about range_cost each (views in plan order)
     std::vector<int> cuts{0};
     double acc = 0.0;
     for (int v = 0; v < G.nv; ++v) {

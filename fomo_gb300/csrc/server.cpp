@@ -10,9 +10,10 @@
 // that arrive meanwhile are admitted into the other slot, so their work
 // overlaps on the device.  A slot's batch marches in view ranges of bounded
 // work (a large view in launches of bounded work), launches with less work
-// first and smaller images first within a launch; each range's cubes download
-// as soon as it is done and its requests complete then, without waiting for the
-// rest of the batch.  Each slot has a high- and a default-priority stream: a
+// first and within a launch the views searched one ray per warp (coarse pixels)
+// before those searched as blocks of rays, smaller images first among either;
+// each range's cubes download as soon as it is done and its requests complete
+// then, without waiting for the rest of the batch.  Each slot has a high- and a default-priority stream: a
 // batch of small requests only goes on the high-priority one, so its kernels
 // start ahead of a large request's next launch.  Results go
 // device -> pinned staging -> the caller's buffer; each request records

@@ -290,11 +290,11 @@ __device__ __forceinline__ float2 fp32_pair(double v) {
 }
 
 // grid: (1 + chunks of kTabChunk table entries, views): an image side may have more chunks than
-// the 65,535 of the grid's y axis.  Block (0, v) fills the
-// view's scalars, independent chains of FP64 divisions on lanes of their own
-// (on one thread, with the tables after them in the same block: 10 us per launch,
-// an FP64 division taking about 0.7); the others fill the tables of ray x, ray y
-// and LOS positions, one entry per thread, from the extents.
+// the 65,535 of the grid's y axis.  Block (0, v) fills the view's scalars,
+// independent chains of FP64 divisions on lanes of their own (on one thread, with
+// the tables after them in the same block: 10 us per launch, an FP64 division
+// taking about 0.7); the others fill the tables of ray x, ray y and LOS
+// positions, one entry per thread, from the extents.
 constexpr int kTabChunk = 128;
 __global__ void __launch_bounds__(kTabChunk) view_finalize_kernel(ViewDesc* views, double3* ktab, float2* ktf, int ktab_stride) {
   ViewDesc* V = views + blockIdx.y;
