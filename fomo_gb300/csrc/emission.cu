@@ -55,20 +55,6 @@ struct PairTables {
   float2 el[256];      // log10(2) times (biased exponent - 127)
 };
 
-struct Pair {
-  float h, l;
-};
-// s + e = a + b exactly
-__device__ __forceinline__ Pair two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
-  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
-}
-// The float that h + l +- E rounds to; false where the bound cannot tell.
-__device__ __forceinline__ bool pair_round(float h, float l, float E, float& t) {
-  t = __fadd_rn(h, __fadd_rn(l, E));
-  return t == __fadd_rn(h, __fsub_rn(l, E));
-}
-
 // fl(log10 v), v > 0.  v = 2^e m, log10 v = e log10 2 - log10 c + log10(1 + r) with r = m c
 // - 1, |r| < 2^-7.9: the series' first term as a pair, the rest (below 2^-17)
 // in FP32.  The lower parts stay below 2^-16 and are added with errors of 2^-41 each.

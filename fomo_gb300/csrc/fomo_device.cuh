@@ -93,4 +93,19 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float v) {
   sum = t;
 }
 
+// An unevaluated sum of two FP32 numbers.
+struct Pair {
+  float h, l;
+};
+// s + e = a + b exactly
+__device__ __forceinline__ Pair two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+  return {s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb))};
+}
+// The float that h + l +- E rounds to; false where the bound cannot tell.
+__device__ __forceinline__ bool pair_round(float h, float l, float E, float& t) {
+  t = __fadd_rn(h, __fadd_rn(l, E));
+  return t == __fadd_rn(h, __fsub_rn(l, E));
+}
+
 }  // namespace fomo

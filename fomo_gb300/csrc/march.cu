@@ -1888,7 +1888,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasShade)
   __shared__ BinShared<NL, NB> staged[kWarps];
   const int w = threadIdx.x >> 5;
   RayCtx r;
-  SpectralBins<NL, NB> bins;
+  SpectralBins<NL, NB, true> bins;
   int view = -1;
   while (next_ray(a, ktab, ktab_stride, a.total_items, r, kCtrShade)) {
     const ViewDesc* V = a.views + r.v;
@@ -1898,7 +1898,7 @@ __global__ void __launch_bounds__(kThreads, kMinCtasShade)
     bins.clear();
     walk_runs(a, r, ktab_stride, rings[w],
               [&](int m, int pos, int len) { bins.add(a.snap, V, staged[w], m, pos, len, a.stats); });
-    bins.write(V, LD, (int64_t)r.i * V->nx + r.j);
+    bins.write(V, LD, staged[w], (int64_t)r.i * V->nx + r.j);
   }
 }
 

@@ -152,6 +152,10 @@ constexpr int kBinThreads = 128;
 constexpr int kBinWarps = kBinThreads / 32;
 constexpr int kPixelWhole = 512;   // points of a pixel one warp sums; a pixel with more is summed in pieces of these
 
+// Points per pixel below which the spectra are scaled by FP32 pairs: with more, FP64 hides behind the profiles (0.5M points, 4
+// lines x 128 bins: 12 points a pixel 267 pairs / 308 us FP64, 24 231 / 232, 48 220 / 209).
+constexpr int64_t kPairsBelow = 24;
+
 // Each point's pixel and its place among the pixel's points.
 __global__ void __launch_bounds__(kProjThreads)
     proj_count_kernel(SnapDev snap, const ViewDesc* __restrict__ V, int* __restrict__ count, int2* __restrict__ at) {
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(kProjThreads)
 // One warp per pixel, taken from a queue; a pixel of more than kPixelWhole points is
 // cleared, and its pieces are queued for the second launch (PIECES), which adds them
 // with atomics.
-template <int NL, int NB, bool PIECES>
+template <int NL, int NB, bool PIECES, bool PAIRS>
 __global__ void __launch_bounds__(kBinThreads, 8)
     proj_bin_kernel(SnapDev snap, const ViewDesc* __restrict__ V, const LineDesc* __restrict__ LD, int nlines,
                     const int* __restrict__ first, const int* __restrict__ list, int2* __restrict__ pieces,
@@ -201,7 +205,7 @@ __global__ void __launch_bounds__(kBinThreads, 8)
   const int nqueue = PIECES ? min((int)ctr[kCtrHard], pieces_cap) : npix;
   // pixels per atomic: up to four where each warp of the grid gets several
   const int grab = PIECES ? 1 : max(1, min(4, npix / ((int)gridDim.x * kBinWarps * 4)));
-  SpectralBins<NL, NB> bins;
+  SpectralBins<NL, NB, PAIRS> bins;
   bins.view(V, LD, nlines, sh);
   for (;;) {
     int q0 = 0;
@@ -228,7 +232,7 @@ __global__ void __launch_bounds__(kBinThreads, 8)
         const int m = min(32, e - i);
         bins.add(snap, V, sh, m, lane < m ? __ldg(list + FOMO_IDX(i + lane, snap.n, kSiteProjection)) : -1, 1, nullptr);
       }
-      bins.template write<PIECES>(V, LD, pix);
+      bins.template write<PIECES>(V, LD, sh, pix);
     }
   }
 }
@@ -238,12 +242,12 @@ cudaError_t launch_bins(const ProjScratch& P, SnapDev snap, const ViewDesc* V, c
                         int64_t npix, int sm_count, cudaStream_t s) {
   const int cap = sm_count * 8;
   const int blocks = (int)std::min<int64_t>(cap, (npix + kBinWarps - 1) / kBinWarps);
-  proj_bin_kernel<NL, NB, false><<<blocks, kBinThreads, 0, s>>>(snap, V, LD, nlines, P.first, P.list, P.pieces,
-                                                               P.pieces_cap, P.ctr);
+  const auto kernel = snap.n < kPairsBelow * npix ? proj_bin_kernel<NL, NB, false, true> : proj_bin_kernel<NL, NB, false, false>;
+  kernel<<<blocks, kBinThreads, 0, s>>>(snap, V, LD, nlines, P.first, P.list, P.pieces, P.pieces_cap, P.ctr);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && snap.n > kPixelWhole) {
     const int64_t most = snap.n / kPixelWhole * 2;
-    proj_bin_kernel<NL, NB, true><<<(int)std::min<int64_t>(cap, (most + kBinWarps - 1) / kBinWarps), kBinThreads, 0, s>>>(
+    proj_bin_kernel<NL, NB, true, false><<<(int)std::min<int64_t>(cap, (most + kBinWarps - 1) / kBinWarps), kBinThreads, 0, s>>>(
         snap, V, LD, nlines, P.first, P.list, P.pieces, P.pieces_cap, P.ctr);
     e = cudaGetLastError();
   }

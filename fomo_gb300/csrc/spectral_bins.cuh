@@ -15,6 +15,7 @@ namespace fomo {
 template <int NL, int NB>
 struct __align__(16) BinShared {
   float4 runs[NL][32];
+  float2 scale[NL];         // of the written sums, as an FP32 pair
   float lams[NL][NB * 32];  // lambdaval (nn:200), evaluated in FP64 on the host, stored FP32
 };
 
@@ -27,8 +28,9 @@ struct __align__(16) BinShared {
 // bytes through the shared-memory port, which was the bound (64 views x 4 lines
 // of 256 x 256 x 512 samples: 22.7 ms, L1 at 85 %); a load now serves four points
 // (18.0 ms).  The groups' sums are joined by an exchange that leaves bin `lane`
-// in each lane, and folded into the pixel's Kahan sum.
-template <int NL, int NB>
+// in each lane, and folded into the pixel's Kahan sum.  PAIRS: the sums are scaled
+// by FP32 pairs where that decides their rounding (scaled), else in FP64.
+template <int NL, int NB, bool PAIRS>
 struct SpectralBins {
   float acc[NL][NB], comp[NL][NB], shk[NL];
   const float2* ew[NL];
@@ -43,6 +45,11 @@ struct SpectralBins {
       ew[l] = on ? LD[l].ew : nullptr;
       shk[l] = on ? LD[l].shift_k : 0.0f;
       nw[l] = on ? min(LD[l].nw, NB) : 0;
+      const double scale = on && LD[l].is_dn ? V->scale_dn : V->scale;
+      const float high = __double2float_rn(scale);
+      const bool usable = fabsf(high) > 1e-30f && fabsf(high) < 1e37f;  // else NaN: every value takes FP64
+      if (PAIRS && lane == 0)
+        sh.scale[l] = make_float2(usable ? high : __int_as_float(0x7fffffff), __double2float_rn(__dsub_rn(scale, (double)high)));
 #pragma unroll
       for (int m = 0; m < NB; ++m) {
         if (m < nw[l]) {
@@ -135,15 +142,35 @@ struct SpectralBins {
     __syncwarp();  // the staged points are rewritten by the next batch
   }
 
+  // fl(scale (acc - comp)) in FP64, and from FP32 pairs where their bound (2^-43; they err by less than 2^-44, the FP64
+  // expression by 2^-52) decides the rounding: the same bits.  A Kahan sum's rest is below 2^-22 of it, so three
+  // operations split the difference; 2^-146 in the bound covers what a tiny product's low part loses below the normal
+  // range; an overflow makes the low part NaN, which decides nothing.  FP64 runs at 1/64 of the FP32 rate, and where rays
+  // have few runs the writes were the emission pass's time: 300 x 300 rays, 4 lines x 100 bins, 2.4 / 27 / 86 runs a ray 469 /
+  // 637 / 1491 us in FP64, 250 / 516 / 1450 from pairs.
+  static __device__ __forceinline__ float scaled_f64(double scale, float acc, float comp) {
+    return __double2float_rn(__dmul_rn(scale, __dsub_rn((double)acc, (double)comp)));
+  }
+  static __device__ __forceinline__ float scaled(const double* scale, float2 s, float acc, float comp) {
+    const float v = __fsub_rn(acc, comp), rest = __fsub_rn(__fsub_rn(acc, v), comp);
+    const float p = __fmul_rn(v, s.x);
+    const float low = fmaf(v, s.x, -p) + fmaf(v, s.y, rest * s.x);
+    float out;
+    if (!pair_round(p, low, fmaf(fabsf(p), 1.14e-13f, 1.2e-44f), out))
+      out = acc == 0.0f && s.x == s.x ? p : scaled_f64(*scale, acc, comp);
+    return out;
+  }
+
   // The pixel's spectra, scaled, into the cubes; ATOMIC: added to what is there.
   template <bool ATOMIC = false>
-  __device__ __forceinline__ void write(const ViewDesc* V, const LineDesc* LD, int64_t ray) {
+  __device__ __forceinline__ void write(const ViewDesc* V, const LineDesc* LD, const BinShared<NL, NB>& sh, int64_t ray) {
     const int lane = threadIdx.x & 31, L = V->L;
     const int64_t ncube = (int64_t)V->nx * V->ny * L;
 #pragma unroll
     for (int l = 0; l < NL; ++l) {
       if (nw[l]) {
-        const double scale = LD[l].is_dn ? V->scale_dn : V->scale;
+        const double* at = LD[l].is_dn ? &V->scale_dn : &V->scale;
+        const double scale = PAIRS ? 0.0 : *at;
         float* out = LD[l].out;
         const int wlo = LD[l].wstart, whi = wlo + 32 * nw[l];
         for (int il = lane; !ATOMIC && il < L; il += 32)
@@ -153,7 +180,7 @@ struct SpectralBins {
           const int il = wlo + m * 32 + lane;
           if (m < nw[l] && il < L) {
             // the sum with what its last additions dropped
-            const float v = __double2float_rn(__dmul_rn(scale, __dsub_rn((double)acc[l][m], (double)comp[l][m])));
+            const float v = PAIRS ? scaled(at, sh.scale[l], acc[l][m], comp[l][m]) : scaled_f64(scale, acc[l][m], comp[l][m]);
             if (ATOMIC)
               atomicAdd(out + FOMO_IDX(ray * L + il, ncube, kSiteCube), v);
             else
