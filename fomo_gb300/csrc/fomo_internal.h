@@ -225,7 +225,7 @@ cudaError_t launch_view_finalize(ViewDesc* views, int nviews, double3* ktab, flo
 
 // projection.cu: the projection render of every view of a group with atomics (outputs zeroed beforehand),
 // or of one view by pixel (its outputs are written whole).
-bool projection_by_pixel(int64_t n, int nlines, int max_windows, bool imaging);
+bool projection_by_pixel(int64_t n, int64_t npix, int nlines, int max_windows, bool imaging);
 int projection_pieces(int64_t n);  // capacity of ProjScratch::pieces
 struct ProjScratch {
   int* count;               // npix + 1: points per pixel

@@ -20,8 +20,13 @@
 // takes 276 by pixel.  kProjListed, points x lines x windows: the direct kernel
 // against the list at 0.11M points, 1 line 86 / 106 us, 4 lines of 2 windows 137 /
 // 112 (96 x 96), 147 / 148 (256 x 256); 0.5M points, 1 line of 2 windows 146 / 146,
-// 4 lines 307 / 183; 2M points, 1 line 322 / 204.  Imaging adds one float per
-// point and line and keeps the direct kernel.
+// 4 lines 307 / 183; 2M points, 1 line 322 / 204.  A warp per pixel also has to be
+// worth it: by pixel from 4 points a pixel on for one line, 3 for more.  2M points
+// at 0.5, 1, 2, 3, 6 points a pixel, the direct kernel / the list: 1 line of 64 bins
+// 490 / 1069, 424 / 662, 392 / 426, 380 / 343, 366 / 254; 4 lines of 64 bins 1565 /
+// 2877, 1303 / 1672, 1176 / 984, 1139 / 741, 1102 / 488; 0.5M points, 4 lines of 128
+// bins 804 / 1782, 662 / 1056, 577 / 640, 552 / 489, 533 / 339.  Imaging adds one
+// float per point and line and keeps the direct kernel.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -258,8 +263,8 @@ cudaError_t launch_bins(const ProjScratch& P, SnapDev snap, const ViewDesc* V, c
 
 FOMO_DEFINE_CHECK_READER(check_word_projection)
 
-bool projection_by_pixel(int64_t n, int nlines, int max_windows, bool imaging) {
-  if (imaging || n * nlines * max_windows < kProjListed) return false;
+bool projection_by_pixel(int64_t n, int64_t npix, int nlines, int max_windows, bool imaging) {
+  if (imaging || n * nlines * max_windows < kProjListed || n < (nlines == 1 ? 4 : 3) * npix) return false;
   return max_windows <= (nlines <= 1 ? 8 : 4) && nlines <= 4;
 }
 

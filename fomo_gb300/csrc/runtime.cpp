@@ -1072,9 +1072,11 @@ int plan_batch(fomo_ctx* ctx, const fomo_request* reqs, int nreq, float* const* 
   for (PlanGroup& G : plan->groups) {
     const int64_t n = ctx->snaps[G.snapshot].n;
     const size_t npix = (size_t)G.maxnpix + 1, bytes = projection_list_bytes(n, G.maxnpix);
+    int64_t pixels = 0;  // of all views
+    for (const auto& v : G.vreqs) pixels += (int64_t)reqs[v[0]].nx * reqs[v[0]].ny;
     // (the windows are known after the descriptors are filled: room for the widest lines)
     G.by_pixel = G.method == FOMO_METHOD_PROJECTION && bytes <= room &&
-                 projection_by_pixel(n, G.nl, G.imaging ? 1 : (G.maxL + 31) / 32, G.imaging != 0);
+                 projection_by_pixel(n, pixels / std::max(G.nv, 1), G.nl, G.imaging ? 1 : (G.maxL + 31) / 32, G.imaging != 0);
     if (!G.by_pixel) continue;
     room -= bytes;
     G.o_pcount = L.take(sizeof(int) * npix);

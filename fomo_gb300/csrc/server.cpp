@@ -139,11 +139,11 @@ size_t request_cost(const fomo_request& q) {
 size_t list_cost(fomo_server* S, const fomo_request& q) {
   const auto it = S->ctx->snaps.find(q.snapshot);
   if (q.method != FOMO_METHOD_PROJECTION || it == S->ctx->snaps.end()) return 0;
-  const int64_t n = it->second.n;
+  const int64_t n = it->second.n, npix = (int64_t)q.nx * q.ny;
   const int windows = (q.nlambda + 31) / 32;
   bool listed = false;
-  for (int nl = 1; nl <= 4; ++nl) listed = listed || projection_by_pixel(n, nl, windows, q.nlambda <= 1);
-  return listed ? projection_list_bytes(n, (int64_t)q.nx * q.ny) : 0;
+  for (int nl = 1; nl <= 4; ++nl) listed = listed || projection_by_pixel(n, npix, nl, windows, q.nlambda <= 1);
+  return listed ? projection_list_bytes(n, npix) : 0;
 }
 
 // Requests `ids` of slot sl are complete (their cubes are in pinned staging);
