@@ -1538,7 +1538,10 @@ __global__ void __launch_bounds__(kThreads, kMinCtasBundle)
             if (gathered) (ncand ? st_far : st_nocand) += __popc(~(done | amb) & valid);
           }
         }
-        if (!gathered) over = true;
+        // march_split searches parts of 16 samples at the least: a segment of 16 goes to the lane walks, as from march_search
+        // (1M-point loop, 400^2 x 8: 2660 us through march_split, 975 so)
+        if (!gathered && nseg > 16) over = true;
+        if (!gathered && nseg <= 16) st_split += __popc(valid);
         __syncwarp();  // the candidate lists are rewritten by the next part
         cur += pn;
       }
