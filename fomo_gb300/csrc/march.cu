@@ -2150,6 +2150,8 @@ __device__ __forceinline__ bool box_cells(const GridParams& g, const BoxQ& q, in
 // sample is the dearer way: a cloud of 64^3 points and eight knots, 101 x 102 x 300, queues 281,000 samples at 64 and 1,700
 // at 192, the render takes 1380 and 810 us, and 1150 with both budgets.  A shorter queue gives 1075 (65,536) and 1020 us (32,768)
 // there, but views of 48^2, whose whole queue is of that length, then wait for late long walks (892 -> 945, 960 -> 1080 us).
+// Views of wide boxes (those with a far pass) keep the short budget: their walks are long in rings, which a warp spreads over its
+// lanes (1.4M-point rope, Thomson, 323 x 92 x 72: 3840 us, 5340 with both; 0.2M-point Gaussian cloud, 731 x 18 x 779: 15.6, 18.9 ms).
 constexpr int kLaneBudget = 64, kLaneBudgetLong = 192;
 constexpr unsigned long long kHardShort = 98304;
 
@@ -2850,7 +2852,7 @@ __device__ __forceinline__ void deferred_search(const MarchArgs& a, int kind, in
       unsigned long long hb = 0;
       if (hm && lane == 0) hb = atomicAdd(a.counter + kCtrHard, (unsigned long long)__popc(hm));
       hb = __shfl_sync(kFull, hb, 0);
-      if (hb >= kHardShort) budget = kLaneBudgetLong;
+      if (hb >= kHardShort && !a.far_list) budget = kLaneBudgetLong;
       if (hard) {
         const int64_t slot = (int64_t)hb + __popc(hm & ((1u << lane) - 1u));
         if (slot < a.hard_cap) {
