@@ -2146,14 +2146,15 @@ __device__ __forceinline__ bool box_cells(const GridParams& g, const BoxQ& q, in
 // Rows + points one lane may scan for one sample before a warp takes it.  With warps waiting for samples the deferred pass
 // lasts as long as its longest walk, and a short budget is the faster: deferred / hard pass at 192, 128, 96, 64: 24 views of 64^2
 // to 700^2 pixels one after the other 7.7 / 2.35, 7.2 / 2.40, 7.0 / 2.44, 6.5 / 2.68 ms; range bounds of 32 and 24 points in
-// place of kLaneDense were no better.  Once kHardShort samples are queued (20 for each warp of the hard pass) a warp per
-// sample is the dearer way: a cloud of 64^3 points and eight knots, 101 x 102 x 300, queues 281,000 samples at 64 and 1,700
-// at 192, the render takes 1380 and 810 us, and 1150 with both budgets.  A shorter queue gives 1075 (65,536) and 1020 us (32,768)
-// there, but views of 48^2, whose whole queue is of that length, then wait for late long walks (892 -> 945, 960 -> 1080 us).
-// Views of wide boxes (those with a far pass) keep the short budget: their walks are long in rings, which a warp spreads over its
-// lanes (1.4M-point rope, Thomson, 323 x 92 x 72: 3840 us, 5340 with both; 0.2M-point Gaussian cloud, 731 x 18 x 779: 15.6, 18.9 ms).
-constexpr int kLaneBudget = 64, kLaneBudgetLong = 192;
-constexpr unsigned long long kHardShort = 98304;
+// place of kLaneDense were no better.  With many samples queued a warp for each is the dearer way where lanes could have ended
+// their walks soon: a warp that sees the queue pass kHardLong goes on with kLaneBudgetLong, and back to a short one for good
+// where a quarter of a batch runs out of that too.  64^3 points and eight knots, 101 x 102 x 300: 281,000 samples
+// queued at 64 and 1,700 at 192, the render 1380 and 810 us, 950 so; 0.4M-point Gaussian cloud, 83 x 77 x 365: 2340, 850, 1040.  Views
+// of wide boxes (those with a far pass) walk longer in empty rings, which a warp spreads over its lanes: there the queue has to
+// be kHardLongWide long (8,192 for all: 40 x 129 x 169 through a rope 672 -> 749 us), and Thomson views keep the short
+// budget (96^2 681 -> 695 us).
+constexpr int kLaneBudget = 64, kLaneBudgetLong = 192, kLaneBudgetFinal = 63;  // (63: short, and not to be changed)
+constexpr unsigned long long kHardLong = 8192, kHardLongWide = 98304;
 
 // Nearest point strictly inside box q, searched by this lane alone: sorted
 // position and original index, or -1 when the box holds no point.  With
@@ -2852,7 +2853,11 @@ __device__ __forceinline__ void deferred_search(const MarchArgs& a, int kind, in
       unsigned long long hb = 0;
       if (hm && lane == 0) hb = atomicAdd(a.counter + kCtrHard, (unsigned long long)__popc(hm));
       hb = __shfl_sync(kFull, hb, 0);
-      if (hb >= kHardShort && !a.far_list) budget = kLaneBudgetLong;
+      const int nh = __popc(hm), nw = min(32, nsamp - t0);
+      if (budget == kLaneBudgetLong)
+        budget = 4 * nh > nw && nw >= 16 ? kLaneBudgetFinal : budget;
+      else if (budget == kLaneBudget && nh && hb >= (a.far_list ? kHardLongWide : kHardLong) && !a.s2)
+        budget = kLaneBudgetLong;
       if (hard) {
         const int64_t slot = (int64_t)hb + __popc(hm & ((1u << lane) - 1u));
         if (slot < a.hard_cap) {

@@ -21,7 +21,7 @@ def _knots(side, share, seed, width):
 
 
 def test_long_hard_queue():
-    """Wide knots seen in a small image: most of the open samples lie in dense cells.  Once 98,304 samples are queued a
+    """Wide knots seen in a small image: most of the open samples lie in dense cells.  Once 8,192 samples are queued a
     lane's walk has the longer budget (192, at which 1,700 of these samples are hard): each of the 152 x 32 warps adds at
     most 32 samples more before it sees that.  With the short budget throughout 281,000 are queued."""
     s = _knots(64, 0.3, seed=3, width=0.5)
@@ -34,4 +34,4 @@ def test_long_hard_queue():
         hard = ctx.profile_read()[1]["hard"]
     _, want, _ = oracle.nn_render(s, eps, w, t.lambda0, 0.5, 0.2, 101, 102, 300, 4, 1e5, want_idx=True)
     np.testing.assert_array_equal(idx, want)
-    assert hard <= 98304 + 32 * 32 * 152 + 1700
+    assert hard <= 8192 + 32 * 32 * 152 + 1700
